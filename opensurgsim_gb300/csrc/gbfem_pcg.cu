@@ -160,7 +160,8 @@ __device__ int lower_bound_warp(const int* __restrict__ arr, int L, int R, int k
 		const int i = L + (lane + 1) * step - 1;
 		const bool pred = (i < R) ? (__ldg(&arr[i]) >= key) : true;
 		const unsigned m = __ballot_sync(kFull, pred);
-		const int k = __ffs(m) - 1;  // m != 0: the last probe is at or past R - 1
+		if (m == 0) return R;  // R - L is a multiple of 32, the last probe is R - 1, and every entry is below key
+		const int k = __ffs(m) - 1;
 		const int iPrev = L + k * step - 1;
 		const int iK = L + (k + 1) * step - 1;
 		L = (k == 0) ? L : iPrev + 1;
