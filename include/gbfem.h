@@ -138,7 +138,8 @@ typedef struct gbfem_stats
 /* Flags for gbfem_step. */
 #define GBFEM_STEP_TIME_PHASES 1u   /* record per-phase device times (adds events) */
 #define GBFEM_STEP_KEEP_SYSTEM 2u   /* keep the full S / rhs / f of the last solve for export */
-#define GBFEM_STEP_TIME_KERNELS 4u  /* time every CG matrix-vector launch with CUDA events */
+#define GBFEM_STEP_TIME_KERNELS 4u  /* time every CG matrix-vector launch with CUDA events (a single FP64 body
+                                       then solves with a launch per product instead of resident) */
 #define GBFEM_STEP_GRAPH 8u         /* mixed form or batch, one Newton iteration: capture the step into a CUDA graph
                                        once and launch it nsteps times with no host round trip between
                                        steps (statistics and the finiteness check are read at the end,
@@ -223,8 +224,10 @@ GBFEM_API gbfem_status gbfem_set_solver_params(gbfem_handle h, int32_t newton_ma
  *   GBFEM_CG_ONE_PHASE: one phase an iteration (Chronopoulos and Gear's recurrences, both dot
  *     products from one reduction): half the phases, larger neighbour records;
  *   GBFEM_CG_FP64: FP64 batches (their only schedule).
- * Without autotuning a handle starts in GBFEM_CG_ONE_PHASE when its system has at most 64 chunks of
- * 32 rows per SM (a few per warp: phases wait on latency), else in GBFEM_CG_TWO_PHASE.
+ * GBFEM_CG_ONE_PHASE and GBFEM_CG_FP64 run resident (every system's matrix in shared memory, CTAs per SM and
+ * refresh weight without effect) where the systems fit, else in the persistent kernel. Without
+ * autotuning a handle starts in GBFEM_CG_ONE_PHASE when its solve is resident or its system has at most 64
+ * chunks of 32 rows per SM (a few per warp: phases wait on latency), else in GBFEM_CG_TWO_PHASE.
  * gbfem_set_tuning's cg_schedule -1 keeps the handle's current schedule. */
 #define GBFEM_CG_TWO_PHASE 0
 #define GBFEM_CG_FP64 1
@@ -285,8 +288,7 @@ GBFEM_API gbfem_status gbfem_rollout_backward(gbfem_handle h, const double* lxT,
  * dofs and states are concatenated in mesh order; every mesh keeps its own CG scalars and
  * convergence test, and one persistent launch solves all of them: in the mixed form its FP32 CG with
  * FP64 refreshes; in the FP64 form (GBFEM_PRECISION_FP64) every mesh's Eigen CG in FP64 (the same
- * iteration and stopping rule as a single FP64 handle, which solves with separate launches per
- * iteration), after the FP64 element update and assembly. Both take GBFEM_STEP_GRAPH and the
+ * iteration and stopping rule as a single FP64 handle), after the FP64 element update and assembly. Both take GBFEM_STEP_GRAPH and the
  * autotuner (CTAs per SM of the solve). gbfem_step, gbfem_get_state, gbfem_set_velocities ... act on
  * the batch. */
 GBFEM_API gbfem_status gbfem_batch_create(int32_t count, const gbfem_mesh_desc* meshes, const gbfem_params* params,

@@ -16,6 +16,7 @@
 #include "../../include/gbfem.h"
 #include "gbfem_internal.h"
 #include "gbfem_pcg.h"
+#include "gbfem_plan.h"
 
 using namespace gbfem;
 
@@ -189,6 +190,21 @@ struct gbfem_handle_s
 	DevBuf<PcgGlobal> d_pcgGlobal;
 	SegCtl* h_seg = nullptr;
 	int pcgGrid = 0;
+	// Resident CG (gbfem_res.cu): the plan of the handle's own solves, its device copies, mailboxes and
+	// exchanged rows.
+	ResPlan res;
+	DevBuf<ResPart> d_resParts;
+	DevBuf<int> d_resHalo, d_resWarp, d_resList;
+	DevBuf<int2> d_resTasks;
+	DevBuf<uint16_t> d_resCol;
+	DevBuf<ResWord> d_resMail, d_resRows;
+	DevBuf<ResCtl> d_resCtl;
+	size_t resSmem = 0;
+	int resBudget = 0;
+	int resForm() const { return res.ok ? res.form : (mixed() ? kResMixed : kResF64); }
+	DevBuf<float4> d_resOwn;  // kResMixedFar: p and x_delta of every row
+	// Whether a solve now runs resident: FP64 whenever a plan fits, the mixed form in its one-phase schedule.
+	bool resident() const { return res.ok && (!mixed() || cgSchedule == kPcgMixed1); }
 	// segments (meshes of a batch): node and tet ranges, chunk ranges
 	std::vector<int> segNode{0}, segTet{0};
 	std::vector<double> segStats;  // per segment over the last gbfem_step: iterations, refreshes, converged, residual
@@ -321,6 +337,13 @@ struct gbfem_handle_s
 		for (auto* b : {&d_rcol, &d_segChunk, &d_cumW, &d_segMaxIter}) b->free();
 		d_slots.free();
 		d_acc.free();
+		d_resParts.free();
+		for (auto* b : {&d_resHalo, &d_resWarp, &d_resList}) b->free();
+		d_resTasks.free();
+		d_resCol.free();
+		for (auto* b : {&d_resMail, &d_resRows}) b->free();
+		d_resOwn.free();
+		d_resCtl.free();
 		for (auto* b : {&d_mcgVec, &d_mcgPart, &d_Re, &d_Wn, &d_xprev}) b->free();
 		d_mcgCtl.free();
 		if (h_mcgCtl) cudaFreeHost(h_mcgCtl);
@@ -395,6 +418,19 @@ cudaError_t raise_pcg_smem_limit(size_t bytes, int form)
 	return e;
 }
 
+// The same for the resident solve.
+cudaError_t raise_res_smem_limit(size_t bytes, int form)
+{
+	static std::mutex mu;
+	static size_t current[kResForms] = {};
+	std::lock_guard<std::mutex> lock(mu);
+	size_t& c = current[form];
+	if (bytes <= std::max<size_t>(c, 48 * 1024)) return cudaSuccess;
+	const cudaError_t e = res_set_max_dynamic_smem(form, (int)bytes);
+	if (e == cudaSuccess) c = bytes;
+	return e;
+}
+
 // Grid of the persistent solve for `cps` CTAs per SM and the handle's refresh weight rw:
 // G = min(cps * SMs, chunks); the largest share of a CTA in chunks (its shared-memory partials) is
 // bounded from the chunk weights: a weighted share holds fewer than tot / (G wmin) + 1 chunks (tot at
@@ -460,6 +496,160 @@ gbfem_status rebuild_hex_operators(gbfem_handle h)
 	GB_CUDA(h, cudaGetLastError());
 	GB_CUDA(h, cudaStreamSynchronize(s));  // before the scratch is released
 	h->linearReady = false;
+	return GBFEM_OK;
+}
+
+// SELL-32 layout of the block matrix under one order of the rows.
+struct SellOrder
+{
+	std::vector<int> perm, segChunk;          // row position -> node (-1 on padding rows); first chunk of each segment
+	std::vector<int> off, scol, rcol;         // chunk offsets; column of each slot as a node and as a row position
+	std::vector<int> sellBase;                // first value of each block of the adjacency
+};
+
+// Orders the rows of every segment by block count (descending; SELL chunks of 32), in node order or
+// (compact) by compact shares of the resident CG, builds the layout and, when `resident`, plans the handle's
+// resident solves (h->res: none where a share's vectors do not fit in an SM's shared memory). A segment is
+// padded to a multiple of 32 rows, so no chunk straddles two.
+gbfem_status order_rows(gbfem_handle h, const double* X, bool compact, bool resident, const std::vector<double>& cost,
+						SellOrder& o)
+{
+	const int nseg = (int)h->segNode.size() - 1, N = h->N;
+	h->res = ResPlan();
+	const int form = h->resForm();
+	auto degree = [&](int I) { return h->adjPtr[I + 1] - h->adjPtr[I]; };
+	std::vector<long long> segWeight(nseg);
+	std::vector<int> segChunks(nseg);
+	for (int sg = 0; sg < nseg; ++sg)
+	{
+		segChunks[sg] = (h->segNode[sg + 1] - h->segNode[sg] + 31) / 32;
+		segWeight[sg] = (h->adjPtr[h->segNode[sg + 1]] - h->adjPtr[h->segNode[sg]]) / 32 + 1 + 4LL * segChunks[sg];
+	}
+	const std::vector<int> width = res_widths(form, compact ? 1.7 : 4.0, segWeight, segChunks, h->smCount, h->resBudget);
+	std::vector<std::vector<int>> cut(nseg);
+	o.perm.clear();
+	o.segChunk.assign(nseg + 1, 0);
+	for (int sg = 0; sg < nseg; ++sg)
+	{
+		const int n0 = h->segNode[sg], n1 = h->segNode[sg + 1], nc = segChunks[sg], g = width[sg];
+		const double* Xs = X + 3 * (size_t)n0;
+		std::vector<int> rows(n1 - n0);
+		for (int i = n0; i < n1; ++i) rows[i - n0] = i;
+		o.segChunk[sg + 1] = o.segChunk[sg] + nc;
+		if (resident && compact && g > 1 && nc >= 4 * g)
+		{
+			// Shares of at least four chunks: boxes, rows by degree inside each (one chunk a share mixes degrees).
+			std::vector<int> w(n1 - n0);
+			for (int i = n0; i < n1; ++i) w[i - n0] = degree(i) + 4;
+			int c = o.segChunk[sg];
+			cut[sg].assign(1, c);
+			for (std::vector<int>& part : res_node_parts(Xs, w, g))
+			{
+				for (int& i : part) i += n0;
+				std::sort(part.begin(), part.end(),
+						  [&](int a, int b) { return degree(a) != degree(b) ? degree(a) > degree(b) : a < b; });
+				part.resize((part.size() + 31) / 32 * 32, -1);
+				o.perm.insert(o.perm.end(), part.begin(), part.end());
+				cut[sg].push_back(c += (int)part.size() / 32);
+			}
+			continue;
+		}
+		if (resident && compact)
+		{
+			// Smaller shares: chunks of one degree, taken along a space-filling curve so that a chunk is compact.
+			const std::vector<uint32_t> key = res_curve_keys(Xs, n1 - n0);
+			std::sort(rows.begin(), rows.end(), [&](int a, int b) {
+				if (degree(a) != degree(b)) return degree(a) > degree(b);
+				return key[a - n0] != key[b - n0] ? key[a - n0] < key[b - n0] : a < b;
+			});
+		}
+		else
+			std::stable_sort(rows.begin(), rows.end(), [&](int a, int b) { return degree(a) > degree(b); });
+		rows.resize((rows.size() + 31) / 32 * 32, -1);
+		if (!resident)
+		{
+			o.perm.insert(o.perm.end(), rows.begin(), rows.end());
+			continue;
+		}
+		// Chunks in an order whose contiguous ranges are compact in space.
+		std::vector<double> centroid(3 * (size_t)nc, 0.0);
+		std::vector<int> weight(nc);
+		for (int c = 0; c < nc; ++c)
+		{
+			int count = 0;
+			for (int l = 0; l < 32 && rows[32 * c + l] >= 0; ++l, ++count)
+				for (int k = 0; k < 3; ++k) centroid[3 * (size_t)c + k] += X[3 * (size_t)rows[32 * c + l] + k];
+			for (int k = 0; k < 3; ++k) centroid[3 * (size_t)c + k] /= count;
+			weight[c] = res_chunk_weight(degree(rows[32 * c]));
+		}
+		for (int c : res_chunk_order(centroid, weight))
+			o.perm.insert(o.perm.end(), rows.begin() + 32 * c, rows.begin() + 32 * (c + 1));
+	}
+	const int nrows = (int)o.perm.size(), nchunks = nrows / 32;
+	std::vector<int> iperm(N, -1);
+	o.off.assign(nchunks + 1, 0);
+	o.sellBase.assign(h->nb, 0);
+	for (int rs = 0; rs < nrows; ++rs)
+		if (o.perm[rs] >= 0) iperm[o.perm[rs]] = rs;
+	for (int c = 0; c < nchunks; ++c)
+	{
+		int w = 0;
+		for (int l = 0; l < 32; ++l)
+			if (o.perm[32 * c + l] >= 0) w = std::max(w, degree(o.perm[32 * c + l]));
+		o.off[c + 1] = o.off[c] + w;
+	}
+	const int64_t sellSlots = 32LL * o.off[nchunks];
+	if (sellSlots * 9 > INT32_MAX) return fail(h, GBFEM_INVALID_ARG, "matrix exceeds int32 indices");
+	// Column of each slot as a node id (dof-space vectors) and as a row position (row-space vectors).
+	// Padding slots point at the row itself with zero values.
+	o.scol.assign(sellSlots, 0);
+	o.rcol.assign(sellSlots, 0);
+	for (int rs = 0; rs < nrows; ++rs)
+	{
+		const int I = o.perm[rs], c = rs >> 5, lane = rs & 31;
+		const int deg = I >= 0 ? degree(I) : 0;
+		for (int t = 0; t < o.off[c + 1] - o.off[c]; ++t)
+		{
+			const int k = o.off[c] + t;
+			const int J = (t < deg) ? h->adj[h->adjPtr[I] + t] : (I >= 0 ? I : o.perm[32 * c]);
+			o.scol[(size_t)k * 32 + lane] = J;
+			o.rcol[(size_t)k * 32 + lane] = (t < deg) ? iperm[J] : rs;
+			if (t < deg) o.sellBase[h->adjPtr[I] + t] = k * 288 + lane;
+		}
+	}
+	for (int64_t k = 0; k < sellSlots; ++k)  // host-side bounds check of every index the kernels follow
+		if (o.scol[k] < 0 || o.scol[k] >= N || o.rcol[k] < 0 || o.rcol[k] >= nrows)
+			return fail(h, GBFEM_CUDA_ERROR, "internal error: SELL index out of range");
+	if (!resident) return GBFEM_OK;
+	for (int sg = 0; sg < nseg; ++sg)
+		if (cut[sg].empty()) cut[sg] = res_cut(o.off, o.segChunk[sg], o.segChunk[sg + 1], width[sg]);
+	h->res = res_plan(form, cut, o.off, o.rcol, cost, h->smCount, h->resBudget);
+	if (!h->res.ok && form == kResMixed) h->res = res_plan(kResMixedFar, cut, o.off, o.rcol, cost, h->smCount, h->resBudget);
+	return GBFEM_OK;
+}
+
+gbfem_status upload_resident(gbfem_handle h, const std::vector<int>& off)
+{
+	cudaStream_t s = h->stream;
+	const ResPlan& r = h->res;
+	const int form = h->resForm();
+	GB_CUDA(h, h->d_resParts.upload(r.parts.data(), r.parts.size(), s));
+	GB_CUDA(h, h->d_resTasks.upload(r.tasks.data(), r.tasks.size(), s));
+	GB_CUDA(h, h->d_resHalo.upload(r.halo.data(), r.halo.size(), s));
+	GB_CUDA(h, h->d_resWarp.upload(r.chunkWarp.data(), r.chunkWarp.size(), s));
+	GB_CUDA(h, h->d_resList.upload(r.chunkList.data(), r.chunkList.size(), s));
+	GB_CUDA(h, h->d_resCol.upload(r.lcol.data(), r.lcol.size(), s));
+	GB_CUDA(h, h->d_resMail.alloc(r.mailWords));
+	GB_CUDA(h, cudaMemsetAsync(h->d_resMail.p, 0, sizeof(ResWord) * r.mailWords, s));
+	const size_t rows = (size_t)res_row_words(form) * h->nrows;
+	GB_CUDA(h, h->d_resRows.alloc(rows));
+	GB_CUDA(h, cudaMemsetAsync(h->d_resRows.p, 0, sizeof(ResWord) * rows, s));
+	if (form == kResMixedFar) GB_CUDA(h, h->d_resOwn.alloc(2 * (size_t)h->nrows));
+	GB_CUDA(h, h->d_resCtl.alloc(1));
+	GB_CUDA(h, cudaMemsetAsync(h->d_resCtl.p, 0, sizeof(ResCtl), s));
+	h->resSmem = res_smem(r, form, off, h->resBudget);
+	GB_CUDA(h, raise_res_smem_limit(h->resSmem, form));
+	GB_CUDA(h, cudaStreamSynchronize(s));
 	return GBFEM_OK;
 }
 
@@ -549,56 +739,48 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 	// block count (descending, stable); each segment is padded to a multiple of 32 rows so that a
 	// chunk of 32 rows never straddles two segments. perm[row] = node id, -1 on padding rows.
 	const int nseg = (int)h->segNode.size() - 1;
-	std::vector<int> perm, chunkSeg, segChunk(nseg + 1, 0);
+	GB_CUDA(h, cudaDeviceGetAttribute(&h->smCount, cudaDevAttrMultiProcessorCount, h->device));
+	int smemSM = 0;
+	GB_CUDA(h, cudaDeviceGetAttribute(&smemSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device));
+	h->resBudget = (smemSM - 2048) / 128 * 128;  // one CTA an SM: less its reserved 1 KB and the kernel's static part
+	// Expected iterations of a system grow with the cells a wave crosses in a step: sqrt(E / rho) / size.
+	std::vector<double> cost(nseg, 1.0);
+	for (int sg = 0; sg < nseg && nseg > 1; ++sg)
+	{
+		double sum = 0.0;
+		const int e0 = h->segTet[sg], e1 = h->segTet[sg + 1];
+		for (int e = e0; e < e1; ++e)
+			sum += std::sqrt(m->young_modulus[e] / m->mass_density[e]) /
+				   std::max(std::cbrt(std::fabs(elemMass[e] / m->mass_density[e])), 1e-300);
+		cost[sg] = 300.0 + sum / std::max(1, e1 - e0);
+	}
+	// The rows' order. The mixed form's FP32 sums round by chunk, and the next step's FP32 element update turns
+	// the last bits of a solution into 1e-9 of its velocities: up to these sizes mixed systems keep the
+	// chunks of rows in node order that the persistent solves use, and the resident solve gives the one-phase
+	// schedule's result bit for bit; batches that had the two-phase schedule keep that too. Larger systems take
+	// the rows of a share from one compact box, as FP64 systems do: the halo is a half to a third
+	// (50,653 nodes on 152 CTAs: 4.1 local rows an own row in node order, 1.8 in boxes; a batch of 687,000
+	// nodes does not fit in node order at all, and its solve takes 5.7 ms in boxes, 15.4 two-phase).
+	SellOrder so;
+	int chunks = 0;
+	for (int sg = 0; sg < nseg; ++sg) chunks += (h->segNode[sg + 1] - h->segNode[sg] + 31) / 32;
+	const bool nodeOrder = h->mixed() && chunks <= (nseg == 1 ? 1024 : 16384);
+	bool resident = !nodeOrder || chunks <= kOnePhaseChunksPerSlot * 4 * h->smCount;
+	// A system of eight times the chip's shared memory reads nearly all of its matrix from L2 and HBM in every
+	// product, which the other solves do with more loads in flight (63^3 hexahedra, mixed, 269 MB: 3.3 ms
+	// resident, 3.5 not).
 	for (int sg = 0; sg < nseg; ++sg)
 	{
-		const int n0 = h->segNode[sg], n1 = h->segNode[sg + 1];
-		std::vector<int> rows(n1 - n0);
-		for (int i = n0; i < n1; ++i) rows[i - n0] = i;
-		std::stable_sort(rows.begin(), rows.end(), [&](int a, int b) {
-			return (h->adjPtr[a + 1] - h->adjPtr[a]) > (h->adjPtr[b + 1] - h->adjPtr[b]);
-		});
-		rows.resize((rows.size() + 31) / 32 * 32, -1);
-		perm.insert(perm.end(), rows.begin(), rows.end());
-		for (size_t c = 0; c < rows.size() / 32; ++c) chunkSeg.push_back(sg);
-		segChunk[sg + 1] = (int)chunkSeg.size();
+		const int64_t blocks = h->adjPtr[h->segNode[sg + 1]] - h->adjPtr[h->segNode[sg]];
+		if (blocks * (h->mixed() ? 38 : 74) > 8LL * h->smCount * smemSM) resident = false;
 	}
-	const int nrows = (int)perm.size();
-	const int nchunks = nrows / 32;
-	std::vector<int> off(nchunks + 1, 0), iperm(N, -1), sellBase(h->nb);
-	for (int rs = 0; rs < nrows; ++rs)
-		if (perm[rs] >= 0) iperm[perm[rs]] = rs;
-	for (int c = 0; c < nchunks; ++c)
-	{
-		int w = 0;
-		for (int l = 0; l < 32; ++l)
-		{
-			const int I = perm[32 * c + l];
-			if (I >= 0) w = std::max(w, h->adjPtr[I + 1] - h->adjPtr[I]);
-		}
-		off[c + 1] = off[c] + w;
-	}
+	gbfem_status ost = order_rows(h, X, !nodeOrder, resident, cost, so);
+	if (ost == GBFEM_OK && resident && !h->res.ok) ost = order_rows(h, X, false, false, cost, so);
+	if (ost != GBFEM_OK) return ost;
+	std::vector<int>&perm = so.perm, &segChunk = so.segChunk, &off = so.off, &scol = so.scol, &rcol = so.rcol,
+					&sellBase = so.sellBase;
+	const int nrows = (int)perm.size(), nchunks = nrows / 32;
 	const int64_t sellSlots = 32LL * off[nchunks];
-	if (sellSlots * 9 > INT32_MAX) return fail(h, GBFEM_INVALID_ARG, "matrix exceeds int32 indices");
-	// Column of each slot as a node id (FP64 form, dof-space vectors) and as a row position (mixed
-	// form, row-space vectors). Padding slots point at the row itself with zero values.
-	std::vector<int> scol(sellSlots, 0), rcol(sellSlots, 0);
-	for (int rs = 0; rs < nrows; ++rs)
-	{
-		const int I = perm[rs], c = rs >> 5, lane = rs & 31;
-		const int deg = (I >= 0) ? h->adjPtr[I + 1] - h->adjPtr[I] : 0;
-		for (int t = 0; t < off[c + 1] - off[c]; ++t)
-		{
-			const int k = off[c] + t;
-			const int J = (t < deg) ? h->adj[h->adjPtr[I] + t] : (I >= 0 ? I : perm[32 * c]);
-			scol[(size_t)k * 32 + lane] = J;
-			rcol[(size_t)k * 32 + lane] = (t < deg) ? iperm[J] : rs;
-			if (t < deg) sellBase[h->adjPtr[I] + t] = k * 288 + lane;
-		}
-	}
-	for (int64_t k = 0; k < sellSlots; ++k)  // host-side bounds check of every index the kernels follow
-		if (scol[k] < 0 || scol[k] >= N || rcol[k] < 0 || rcol[k] >= nrows)
-			return fail(h, GBFEM_CUDA_ERROR, "internal error: SELL index out of range");
 	h->sellSlots = sellSlots;
 	h->nrows = nrows;
 	h->nchunks = nchunks;
@@ -710,6 +892,11 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 	GB_CUDA(h, h->d_perm.upload(perm.data(), perm.size(), s));
 	GB_CUDA(h, h->d_off.upload(off.data(), off.size(), s));
 	GB_CUDA(h, h->d_sellcol.upload(scol.data(), scol.size(), s));
+	if (h->res.ok)
+	{
+		gbfem_status rst = upload_resident(h, off);
+		if (rst != GBFEM_OK) return rst;
+	}
 	if (h->persistent())
 	{
 		GB_CUDA(h, h->d_rcol.upload(rcol.data(), rcol.size(), s));
@@ -748,10 +935,14 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 	}
 	// The persistent solve's control structures (mixed form, FP64 batches): per-segment CG state, the
 	// chunk weights its partition balances, the grid and the per-segment iteration caps.
-	auto setup_persistent = [&]() -> gbfem_status {
+	if (h->persistent() || h->res.ok)
+	{
 		GB_CUDA(h, h->d_seg.alloc(nseg));
 		GB_CUDA(h, h->d_pcgGlobal.alloc(1));
+		GB_CUDA(h, cudaMemsetAsync(h->d_pcgGlobal.p, 0, sizeof(PcgGlobal), s));
 		GB_CUDA(h, cudaMallocHost(&h->h_seg, sizeof(SegCtl) * nseg));
+	}
+	auto setup_persistent = [&]() -> gbfem_status {
 		// Persistent grid: as many co-resident CTAs as fit, at most 4 per SM. The kernel splits the
 		// chunks of the segments still iterating over the CTAs itself; the host bounds the largest
 		// share (shared-memory partials) from the chunk weights.
@@ -764,14 +955,13 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 			if ((int64_t)cumW[c] + w > INT32_MAX) return fail(h, GBFEM_INVALID_ARG, "matrix too large for the persistent solve");
 			cumW[c + 1] = cumW[c] + w;
 		}
-		GB_CUDA(h, cudaDeviceGetAttribute(&h->smCount, cudaDevAttrMultiProcessorCount, h->device));
 		h->chunkWeightTotal = cumW[nchunks];
 		h->chunkWeightMin = std::max(1, wmin);
 		// CG schedule until the autotuner or gbfem_set_tuning picks one: one grid phase an iteration
 		// where a phase leaves each warp a few chunks (its phases wait on latency; one 1.28M-tet mesh,
 		// 8,458 chunks: 17.2 vs 22.9 ms a solve), two phases where phases stream many chunks a warp
 		// (64 meshes, 19,549 chunks: 15.7 vs 16.3 ms; 256 meshes: 41.3 vs 53.1 ms).
-		h->cgSchedule = (nchunks <= kOnePhaseChunksPerSlot * 4 * h->smCount) ? kPcgMixed1 : kPcgMixed2;
+		h->cgSchedule = (h->res.ok || nchunks <= kOnePhaseChunksPerSlot * 4 * h->smCount) ? kPcgMixed1 : kPcgMixed2;
 		gbfem_status cst = GBFEM_INVALID_ARG;
 		std::string why;
 		for (int cps = 4; cps >= 1 && cst != GBFEM_OK; --cps)
@@ -808,9 +998,9 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 		if (h->batched())
 		{
 			// FP64 batch: the persistent FP64 CG's row-space vectors; z and p of a row in one 64-byte record.
-			const size_t nr = 3 * (size_t)nrows;
+			const size_t nr = h->res.ok ? 0 : 3 * (size_t)nrows;
 			for (DevBuf<double>* b : {&h->d_invd64, &h->d_q64, &h->d_r64, &h->d_x64}) GB_CUDA(h, b->alloc(nr));
-			for (DevBuf<double>* b : {&h->d_zA64, &h->d_zB64}) GB_CUDA(h, b->alloc(8 * (size_t)nrows));
+			for (DevBuf<double>* b : {&h->d_zA64, &h->d_zB64}) GB_CUDA(h, b->alloc(h->res.ok ? 0 : 8 * (size_t)nrows));
 			gbfem_status pst = setup_persistent();
 			if (pst != GBFEM_OK) return pst;
 			GB_CUDA(h, cudaStreamSynchronize(s));
@@ -1046,6 +1236,57 @@ gbfem_status run_cg(gbfem_handle h, const double* b, double* x, int maxIter, boo
 	return GBFEM_OK;
 }
 
+// Refresh when |r|^2 has dropped 1e5x (the residual norm ~300x) since the last refresh: FP32 CG keeps
+// several digits of headroom below that, and each refresh is an extra pass in double-float arithmetic.
+// Measured on the 256-mesh batch: 1e-3 -> 1e-5 kept the CG iterations (226.7 / 227.1 per step)
+// and the error against the FP64 path, and cut the step by 7%.
+constexpr double kRefreshDrop = 1e-5;
+
+// One resident solve of every system of the handle (gbfem_res.cu): one launch, no memory set before it.
+gbfem_status enqueue_resident(gbfem_handle h, const double* b, double* x, int maxIter, cudaEvent_t ev0, cudaEvent_t ev1,
+							  bool capturing)
+{
+	cudaStream_t st = h->stream;
+	ResArgs a{};
+	a.parts = h->d_resParts.p;
+	a.tasks = h->d_resTasks.p;
+	a.nTasks = (int)h->res.tasks.size();
+	a.off = h->d_off.p;
+	a.lcol = h->d_resCol.p;
+	a.halo = h->d_resHalo.p;
+	a.chunkWarp = h->d_resWarp.p;
+	a.chunkList = h->d_resList.p;
+	a.perm = h->d_perm.p;
+	// Without an explicit cg_max_iterations every system of a batch or of the mixed form stops at its own
+	// default cap.
+	const bool segCaps = h->persistent() && h->prm.cg_max_iterations <= 0;
+	a.maxIter = segCaps ? h->segMaxIterMax : maxIter;
+	a.segMaxIter = segCaps ? h->d_segMaxIter.p : nullptr;
+	a.smemBudget = (int)h->resSmem;
+	a.tol = h->prm.cg_tolerance;
+	a.drop = kRefreshDrop;
+	a.timeoutNs = kBarrierTimeoutNs;
+	a.mail = h->d_resMail.p;
+	a.rowWords = h->d_resRows.p;
+	a.ctl = h->d_resCtl.p;
+	a.seg = h->d_seg.p;
+	a.err = &h->d_pcgGlobal.p->err;
+	a.b = b;
+	a.x = x;
+	a.val = h->mixed() ? (const void*)h->d_A32.p : h->d_A.p;
+	a.invdiag = h->mixed() ? (const void*)h->d_invdiag32.p : h->d_invdiag.p;
+	a.xhl = reinterpret_cast<float2*>(h->d_x64.p);
+	a.r64 = h->d_r64.p;
+	a.own = h->d_resOwn.p;
+	a.nrows = h->nrows;
+	const unsigned evFlags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
+	if (ev0) GB_CUDA(h, cudaEventRecordWithFlags(ev0, st, evFlags));
+	GB_CUDA(h, res_launch(h->resForm(), h->res.grid, h->resSmem, a, st));
+	if (ev1) GB_CUDA(h, cudaEventRecordWithFlags(ev1, st, evFlags));
+	h->launches += 1;
+	return GBFEM_OK;
+}
+
 // Mixed-precision solve: FP32 CG iterations with reliable FP64 residual refreshes; the host polls
 // the device control block between chunks of iterations.
 // Enqueue one persistent solve on the handle's stream (no host synchronisation; capturable).
@@ -1054,6 +1295,7 @@ gbfem_status run_cg(gbfem_handle h, const double* b, double* x, int maxIter, boo
 gbfem_status enqueue_mixed(gbfem_handle h, const double* b, double* x, int maxIter, cudaEvent_t ev0, cudaEvent_t ev1,
 						   bool capturing = false)
 {
+	if (h->resident()) return enqueue_resident(h, b, x, maxIter, ev0, ev1, capturing);
 	const int nseg = (int)h->segNode.size() - 1;
 	cudaStream_t st = h->stream;
 	GB_CUDA(h, cudaMemsetAsync(h->d_seg.p, 0, sizeof(SegCtl) * nseg, st));
@@ -1066,11 +1308,7 @@ gbfem_status enqueue_mixed(gbfem_handle h, const double* b, double* x, int maxIt
 	a.maxIter = segCaps ? h->segMaxIterMax : maxIter;
 	a.segMaxIter = segCaps ? h->d_segMaxIter.p : nullptr;
 	a.tol = h->prm.cg_tolerance;
-	// Refresh when |r|^2 has dropped 1e5x (the residual norm ~300x) since the last refresh: FP32 CG keeps
-	// several digits of headroom below that, and each refresh is an FP64 pass (9 FP64 FMAs a block).
-	// Measured on the 256-mesh batch: 1e-3 -> 1e-5 kept the CG iterations (226.7 / 227.1 per step)
-	// and the error against the FP64 path, and cut the step by 7%.
-	a.drop = 1e-5;
+	a.drop = kRefreshDrop;
 	a.off = h->d_off.p;
 	a.col = h->d_rcol.p;
 	a.val = h->d_A32.p;
@@ -1136,8 +1374,11 @@ gbfem_status run_mixed(gbfem_handle h, const double* b, double* x, int maxIter, 
 	GB_CUDA(h, cudaMemcpyAsync(&g, h->d_pcgGlobal.p, sizeof(PcgGlobal), cudaMemcpyDeviceToHost, st));
 	GB_CUDA(h, cudaStreamSynchronize(st));
 	if (g.err)
+	{
+		GB_CUDA(h, cudaMemsetAsync(h->d_pcgGlobal.p, 0, sizeof(PcgGlobal), st));
 		return fail(h, GBFEM_CUDA_ERROR, g.err == 1 ? "persistent CG: grid barrier timed out"
 												  : "persistent CG: work share exceeded its shared-memory bound");
+	}
 	if (timeSolve)
 	{
 		float ms = 0;
@@ -1239,6 +1480,7 @@ gbfem_status tune_mixed(gbfem_handle h, const double* xt, const double* vt, doub
 			for (int rw : {1, 2, 3, 4})
 			{
 				if (f64 && rw != kRefreshWeightDefault) continue;  // the FP64 solve has no refreshes
+				if (h->resident() && (cps != 4 || rw != kRefreshWeightDefault)) continue;  // its plan has neither choice
 				h->refreshWeight = rw;
 				if (configure_pcg(h, cps) != GBFEM_OK)
 				{
@@ -1642,10 +1884,11 @@ gbfem_status step_once(gbfem_handle h, double dt, uint32_t flags)
 				if (est != GBFEM_OK) return est;
 			}
 			tm.mark(2);
-			if (h->batched())
+			if (h->batched() || (h->resident() && !timeK))
 			{
-				// FP64 batch: every mesh's Eigen CG in one persistent FP64 launch.
-				if (h->prm.autotune && !h->tuned)
+				// Every system's Eigen CG in one launch. (GBFEM_STEP_TIME_KERNELS asks for the time of each
+				// matrix-vector product of a single body, which the launch-per-iteration solve has.)
+				if (h->batched() && h->prm.autotune && !h->tuned)
 				{
 					gbfem_status tst = tune_mixed(h, xt, vt, dt, c1, c2, maxIter);
 					if (tst != GBFEM_OK) return tst;
@@ -2121,7 +2364,7 @@ gbfem_status gbfem_adjoint_step(gbfem_handle h, double dt, const double* x, cons
 	h->launches += ek + 2;
 	tm.mark(1);
 	bool converged = true;
-	if (h->persistent())
+	if (h->persistent() || h->resident())
 	{
 		gbfem_status st = run_mixed(h, h->d_adjG.p, h->d_mu.p, maxIter, false);
 		if (st != GBFEM_OK) return st;
