@@ -53,6 +53,124 @@ struct DevBuf
 	}
 };
 
+// Dynamic shared memory the resident solve's kernel may use, raised as needed (once per process and form).
+cudaError_t raise_res_smem_limit(size_t bytes, int form)
+{
+	static std::mutex mu;
+	static size_t current[kResForms] = {};
+	std::lock_guard<std::mutex> lock(mu);
+	size_t& c = current[form];
+	if (bytes <= std::max<size_t>(c, 48 * 1024)) return cudaSuccess;
+	const cudaError_t e = res_set_max_dynamic_smem(form, (int)bytes);
+	if (e == cudaSuccess) c = bytes;
+	return e;
+}
+
+// Shared memory of a resident CTA: one CTA an SM, less its reserved 1 KB and the kernel's static part.
+cudaError_t res_budget(int device, int* smCount, int* budget)
+{
+	int smem = 0;
+	cudaError_t e = cudaDeviceGetAttribute(smCount, cudaDevAttrMultiProcessorCount, device);
+	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+	*budget = (smem - 2048) / 128 * 128;
+	return e;
+}
+
+// A plan of the resident CG (gbfem_res.cu) on the device.
+struct ResDevice
+{
+	ResPlan plan;  // without its halo and column lists, which only the device reads
+	int maxRhs = 0;
+	size_t smem = 0;
+	DevBuf<ResPart> parts;
+	DevBuf<int> halo, warp, list;
+	DevBuf<int2> tasks;
+	DevBuf<uint16_t> lcol;
+
+	// rhs: right-hand sides a launch may take. Waits for the copies.
+	cudaError_t upload(ResPlan&& p, const std::vector<int>& off, int budget, int rhs, cudaStream_t s)
+	{
+		plan = std::move(p);
+		maxRhs = rhs;
+		std::vector<int2> t;
+		t.reserve(plan.tasks.size() * rhs);
+		for (int c = 0; c < rhs; ++c)
+			for (const int2& u : plan.tasks) t.push_back(make_int2(u.x, c));
+		cudaError_t e = parts.upload(plan.parts.data(), plan.parts.size(), s);
+		if (e == cudaSuccess) e = tasks.upload(t.data(), t.size(), s);
+		if (e == cudaSuccess) e = halo.upload(plan.halo.data(), plan.halo.size(), s);
+		if (e == cudaSuccess) e = warp.upload(plan.chunkWarp.data(), plan.chunkWarp.size(), s);
+		if (e == cudaSuccess) e = list.upload(plan.chunkList.data(), plan.chunkList.size(), s);
+		if (e == cudaSuccess) e = lcol.upload(plan.lcol.data(), plan.lcol.size(), s);
+		smem = res_smem(plan, plan.form, off, budget);
+		if (e == cudaSuccess) e = raise_res_smem_limit(smem, plan.form);
+		if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+		for (auto* v : {&plan.halo, &plan.chunkWarp, &plan.chunkList}) std::vector<int>().swap(*v);
+		std::vector<uint16_t>().swap(plan.lcol);
+		return e;
+	}
+	void fill(ResArgs& a, int rhs) const
+	{
+		a.parts = parts.p;
+		a.tasks = tasks.p;
+		a.nTasks = (int)plan.tasks.size() * rhs;
+		a.halo = halo.p;
+		a.chunkWarp = warp.p;
+		a.chunkList = list.p;
+		a.lcol = lcol.p;
+		a.smemBudget = (int)smem;
+	}
+	cudaError_t launch(const ResArgs& a, int ctas, cudaStream_t s) const
+	{
+		return res_launch(plan.form, std::min(ctas, a.nTasks), smem, a, s);
+	}
+	void free()
+	{
+		parts.free();
+		for (auto* b : {&halo, &warp, &list}) b->free();
+		tasks.free();
+		lcol.free();
+		plan = ResPlan();
+	}
+};
+
+// What the CTAs of resident launches exchange. The tags of a launch lie above those of every launch before it,
+// so plans of one stream share the words without clearing them.
+struct ResExchange
+{
+	DevBuf<ResWord> mail, rows;
+	DevBuf<ResCtl> ctl;
+	cudaError_t reserve(size_t mailWords, size_t rowWords, cudaStream_t s)
+	{
+		cudaError_t e = cudaSuccess;
+		if (!ctl.p)
+		{
+			e = ctl.alloc(1);
+			if (e == cudaSuccess) e = cudaMemsetAsync(ctl.p, 0, sizeof(ResCtl), s);
+		}
+		for (auto& want : {std::make_pair(&mail, mailWords), std::make_pair(&rows, rowWords)})
+			if (e == cudaSuccess && want.first->n < want.second)
+			{
+				e = cudaStreamSynchronize(s);
+				if (e == cudaSuccess) e = want.first->alloc(want.second);
+				if (e == cudaSuccess) e = cudaMemsetAsync(want.first->p, 0, sizeof(ResWord) * want.second, s);
+			}
+		return e;
+	}
+	void fill(ResArgs& a) const
+	{
+		a.mail = mail.p;
+		a.rowWords = rows.p;
+		a.ctl = ctl.p;
+	}
+	void free()
+	{
+		mail.free();
+		rows.free();
+		ctl.free();
+	}
+};
+
 double det3v(const double* a, const double* b, const double* c)
 {
 	return a[0] * b[1] * c[2] + a[2] * b[0] * c[1] + a[1] * b[2] * c[0] - a[2] * b[1] * c[0] - a[1] * b[0] * c[2] -
@@ -190,19 +308,19 @@ struct gbfem_handle_s
 	DevBuf<PcgGlobal> d_pcgGlobal;
 	SegCtl* h_seg = nullptr;
 	int pcgGrid = 0;
-	// Resident CG (gbfem_res.cu): the plan of the handle's own solves, its device copies, mailboxes and
-	// exchanged rows.
+	// Resident CG (gbfem_res.cu): the plan of the handle's own solves.
 	ResPlan res;
-	DevBuf<ResPart> d_resParts;
-	DevBuf<int> d_resHalo, d_resWarp, d_resList;
-	DevBuf<int2> d_resTasks;
-	DevBuf<uint16_t> d_resCol;
-	DevBuf<ResWord> d_resMail, d_resRows;
-	DevBuf<ResCtl> d_resCtl;
-	size_t resSmem = 0;
+	ResDevice d_res;
+	ResExchange resLink;
 	int resBudget = 0;
 	int resForm() const { return res.ok ? res.form : (mixed() ? kResMixed : kResF64); }
 	DevBuf<float4> d_resOwn;  // kResMixedFar: p and x_delta of every row
+	// Compliance columns: plans by CTAs a column, their exchange, columns and results.
+	std::map<int, ResDevice> colPlans;
+	ResExchange colLink;
+	DevBuf<double> d_colB, d_colX;
+	DevBuf<SegCtl> d_colSeg;
+	DevBuf<PcgGlobal> d_colErr;
 	// Whether a solve now runs resident: FP64 whenever a plan fits, the mixed form in its one-phase schedule.
 	bool resident() const { return res.ok && (!mixed() || cgSchedule == kPcgMixed1); }
 	// segments (meshes of a batch): node and tet ranges, chunk ranges
@@ -337,13 +455,16 @@ struct gbfem_handle_s
 		for (auto* b : {&d_rcol, &d_segChunk, &d_cumW, &d_segMaxIter}) b->free();
 		d_slots.free();
 		d_acc.free();
-		d_resParts.free();
-		for (auto* b : {&d_resHalo, &d_resWarp, &d_resList}) b->free();
-		d_resTasks.free();
-		d_resCol.free();
-		for (auto* b : {&d_resMail, &d_resRows}) b->free();
+		d_res.free();
+		resLink.free();
 		d_resOwn.free();
-		d_resCtl.free();
+		for (auto& p : colPlans) p.second.free();
+		colPlans.clear();
+		colLink.free();
+		d_colB.free();
+		d_colX.free();
+		d_colSeg.free();
+		d_colErr.free();
 		for (auto* b : {&d_mcgVec, &d_mcgPart, &d_Re, &d_Wn, &d_xprev}) b->free();
 		d_mcgCtl.free();
 		if (h_mcgCtl) cudaFreeHost(h_mcgCtl);
@@ -415,19 +536,6 @@ cudaError_t raise_pcg_smem_limit(size_t bytes, int form)
 	if (bytes <= current[form]) return cudaSuccess;
 	const cudaError_t e = pcg_set_max_dynamic_smem(form, (int)bytes);
 	if (e == cudaSuccess) current[form] = bytes;
-	return e;
-}
-
-// The same for the resident solve.
-cudaError_t raise_res_smem_limit(size_t bytes, int form)
-{
-	static std::mutex mu;
-	static size_t current[kResForms] = {};
-	std::lock_guard<std::mutex> lock(mu);
-	size_t& c = current[form];
-	if (bytes <= std::max<size_t>(c, 48 * 1024)) return cudaSuccess;
-	const cudaError_t e = res_set_max_dynamic_smem(form, (int)bytes);
-	if (e == cudaSuccess) c = bytes;
 	return e;
 }
 
@@ -630,26 +738,11 @@ gbfem_status order_rows(gbfem_handle h, const double* X, bool compact, bool resi
 
 gbfem_status upload_resident(gbfem_handle h, const std::vector<int>& off)
 {
-	cudaStream_t s = h->stream;
-	const ResPlan& r = h->res;
-	const int form = h->resForm();
-	GB_CUDA(h, h->d_resParts.upload(r.parts.data(), r.parts.size(), s));
-	GB_CUDA(h, h->d_resTasks.upload(r.tasks.data(), r.tasks.size(), s));
-	GB_CUDA(h, h->d_resHalo.upload(r.halo.data(), r.halo.size(), s));
-	GB_CUDA(h, h->d_resWarp.upload(r.chunkWarp.data(), r.chunkWarp.size(), s));
-	GB_CUDA(h, h->d_resList.upload(r.chunkList.data(), r.chunkList.size(), s));
-	GB_CUDA(h, h->d_resCol.upload(r.lcol.data(), r.lcol.size(), s));
-	GB_CUDA(h, h->d_resMail.alloc(r.mailWords));
-	GB_CUDA(h, cudaMemsetAsync(h->d_resMail.p, 0, sizeof(ResWord) * r.mailWords, s));
-	const size_t rows = (size_t)res_row_words(form) * h->nrows;
-	GB_CUDA(h, h->d_resRows.alloc(rows));
-	GB_CUDA(h, cudaMemsetAsync(h->d_resRows.p, 0, sizeof(ResWord) * rows, s));
+	const int form = h->res.form;
+	GB_CUDA(h, h->resLink.reserve(h->res.mailWords, (size_t)res_row_words(form) * h->nrows, h->stream));
 	if (form == kResMixedFar) GB_CUDA(h, h->d_resOwn.alloc(2 * (size_t)h->nrows));
-	GB_CUDA(h, h->d_resCtl.alloc(1));
-	GB_CUDA(h, cudaMemsetAsync(h->d_resCtl.p, 0, sizeof(ResCtl), s));
-	h->resSmem = res_smem(r, form, off, h->resBudget);
-	GB_CUDA(h, raise_res_smem_limit(h->resSmem, form));
-	GB_CUDA(h, cudaStreamSynchronize(s));
+	GB_CUDA(h, h->d_res.upload(ResPlan(h->res), off, h->resBudget, 1, h->stream));
+	std::vector<uint16_t>().swap(h->res.lcol);
 	return GBFEM_OK;
 }
 
@@ -739,10 +832,7 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 	// block count (descending, stable); each segment is padded to a multiple of 32 rows so that a
 	// chunk of 32 rows never straddles two segments. perm[row] = node id, -1 on padding rows.
 	const int nseg = (int)h->segNode.size() - 1;
-	GB_CUDA(h, cudaDeviceGetAttribute(&h->smCount, cudaDevAttrMultiProcessorCount, h->device));
-	int smemSM = 0;
-	GB_CUDA(h, cudaDeviceGetAttribute(&smemSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device));
-	h->resBudget = (smemSM - 2048) / 128 * 128;  // one CTA an SM: less its reserved 1 KB and the kernel's static part
+	GB_CUDA(h, res_budget(h->device, &h->smCount, &h->resBudget));
 	// Expected iterations of a system grow with the cells a wave crosses in a step: sqrt(E / rho) / size.
 	std::vector<double> cost(nseg, 1.0);
 	for (int sg = 0; sg < nseg && nseg > 1; ++sg)
@@ -772,7 +862,7 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 	for (int sg = 0; sg < nseg; ++sg)
 	{
 		const int64_t blocks = h->adjPtr[h->segNode[sg + 1]] - h->adjPtr[h->segNode[sg]];
-		if (blocks * (h->mixed() ? 38 : 74) > 8LL * h->smCount * smemSM) resident = false;
+		if (blocks * (h->mixed() ? 38 : 74) > 8LL * h->smCount * h->resBudget) resident = false;
 	}
 	gbfem_status ost = order_rows(h, X, !nodeOrder, resident, cost, so);
 	if (ost == GBFEM_OK && resident && !h->res.ok) ost = order_rows(h, X, false, false, cost, so);
@@ -1248,27 +1338,18 @@ gbfem_status enqueue_resident(gbfem_handle h, const double* b, double* x, int ma
 {
 	cudaStream_t st = h->stream;
 	ResArgs a{};
-	a.parts = h->d_resParts.p;
-	a.tasks = h->d_resTasks.p;
-	a.nTasks = (int)h->res.tasks.size();
+	h->d_res.fill(a, 1);
+	h->resLink.fill(a);
 	a.off = h->d_off.p;
-	a.lcol = h->d_resCol.p;
-	a.halo = h->d_resHalo.p;
-	a.chunkWarp = h->d_resWarp.p;
-	a.chunkList = h->d_resList.p;
 	a.perm = h->d_perm.p;
 	// Without an explicit cg_max_iterations every system of a batch or of the mixed form stops at its own
 	// default cap.
 	const bool segCaps = h->persistent() && h->prm.cg_max_iterations <= 0;
 	a.maxIter = segCaps ? h->segMaxIterMax : maxIter;
 	a.segMaxIter = segCaps ? h->d_segMaxIter.p : nullptr;
-	a.smemBudget = (int)h->resSmem;
 	a.tol = h->prm.cg_tolerance;
 	a.drop = kRefreshDrop;
 	a.timeoutNs = kBarrierTimeoutNs;
-	a.mail = h->d_resMail.p;
-	a.rowWords = h->d_resRows.p;
-	a.ctl = h->d_resCtl.p;
 	a.seg = h->d_seg.p;
 	a.err = &h->d_pcgGlobal.p->err;
 	a.b = b;
@@ -1281,7 +1362,7 @@ gbfem_status enqueue_resident(gbfem_handle h, const double* b, double* x, int ma
 	a.nrows = h->nrows;
 	const unsigned evFlags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
 	if (ev0) GB_CUDA(h, cudaEventRecordWithFlags(ev0, st, evFlags));
-	GB_CUDA(h, res_launch(h->resForm(), h->res.grid, h->resSmem, a, st));
+	GB_CUDA(h, h->d_res.launch(a, h->smCount, st));
 	if (ev1) GB_CUDA(h, cudaEventRecordWithFlags(ev1, st, evFlags));
 	h->launches += 1;
 	return GBFEM_OK;
@@ -2117,6 +2198,138 @@ gbfem_status gbfem_batch_create(int32_t count, const gbfem_mesh_desc* meshes, co
 	return create_impl(meshes, count, params, out);
 }
 
+namespace {
+
+// Plan of ncols compliance columns as resident solves side by side, or null where none fits. A few CTAs
+// a column keep more columns going at once, many shorten each: an iteration takes about 6.5 us + 0.07 us a
+// weight of a share (FP64 sums at 64 cycles an instruction), and the columns go in waves. One plan per
+// number of CTAs, at most fifteen in a handle.
+gbfem_status compliance_plan(gbfem_handle h, int ncols, ResDevice** out)
+{
+	*out = nullptr;
+	if (h->batched() || !h->res.ok) return GBFEM_OK;
+	const int form = h->mixed() ? kResF64M : kResF64;
+	const double weight = h->sellSlots / 32 + 4.0 * h->nchunks;
+	struct Choice
+	{
+		double us;
+		int g;
+	};
+	std::vector<Choice> choice;
+	for (int g : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128, 152})
+		if (g <= std::min({h->smCount, h->nchunks, kResMaxGroup}))
+			choice.push_back({std::ceil(ncols / std::floor((double)h->smCount / g)) * (6.5 + 0.07 * weight / g), g});
+	std::stable_sort(choice.begin(), choice.end(), [](const Choice& a, const Choice& b) { return a.us < b.us; });
+	std::vector<int> off, rcol;
+	for (const Choice& c : choice)
+	{
+		auto have = h->colPlans.find(c.g);
+		if (have == h->colPlans.end())
+		{
+			if (off.empty())
+			{
+				// The layout's host copy is gone: read it back.
+				std::vector<int> perm(h->nrows), iperm(h->N, 0);
+				off.resize(h->nchunks + 1);
+				rcol.resize(h->sellSlots);
+				GB_CUDA(h, cudaMemcpyAsync(off.data(), h->d_off.p, sizeof(int) * off.size(), cudaMemcpyDeviceToHost, h->stream));
+				GB_CUDA(h, cudaMemcpyAsync(perm.data(), h->d_perm.p, sizeof(int) * perm.size(), cudaMemcpyDeviceToHost, h->stream));
+				GB_CUDA(h, cudaMemcpyAsync(rcol.data(), h->d_sellcol.p, sizeof(int) * rcol.size(), cudaMemcpyDeviceToHost, h->stream));
+				GB_CUDA(h, cudaStreamSynchronize(h->stream));
+				for (int r = 0; r < h->nrows; ++r)
+					if (perm[r] >= 0) iperm[perm[r]] = r;
+				for (int& r : rcol) r = iperm[r];  // on padding slots any row of the system will do: their values are zero
+			}
+			ResPlan plan = res_plan(form, {res_cut(off, 0, h->nchunks, c.g)}, off, rcol, {1.0}, h->smCount, h->resBudget);
+			ResDevice d;
+			if (plan.ok)
+			{
+				// Columns a launch takes: four waves, at most 256 MB of exchanged rows.
+				const int waves = 4 * (h->smCount / c.g);
+				const int room = (int)std::max<int64_t>(1, ((int64_t)256 << 20) / (48LL * h->nrows));
+				const cudaError_t e = d.upload(std::move(plan), off, h->resBudget, std::min(waves, room), h->stream);
+				if (e != cudaSuccess) d.free();
+				GB_CUDA(h, e);
+			}
+			have = h->colPlans.emplace(c.g, std::move(d)).first;
+		}
+		if (!have->second.plan.ok) continue;
+		*out = &have->second;
+		return GBFEM_OK;
+	}
+	return GBFEM_OK;
+}
+
+// Compliance columns by resident solves; Wn: node rotations or null.
+gbfem_status compliance_resident(gbfem_handle h, ResDevice& d, int ncols, const double* b, double* x, const double* Wn,
+								 int maxIter, int* iterations, bool* allConverged)
+{
+	cudaStream_t s = h->stream;
+	const int n = h->n, most = std::min(d.maxRhs, ncols);
+	const size_t mailStride = d.plan.mailWords, rowStride = (size_t)res_row_words(d.plan.form) * h->nrows;
+	GB_CUDA(h, h->colLink.reserve(mailStride * most, rowStride * most, s));
+	if (h->d_colSeg.n < (size_t)most)
+	{
+		GB_CUDA(h, h->d_colB.alloc((size_t)n * most));
+		GB_CUDA(h, h->d_colX.alloc((size_t)n * most));
+		GB_CUDA(h, h->d_colSeg.alloc(most));
+	}
+	if (!h->d_colErr.p)
+	{
+		GB_CUDA(h, h->d_colErr.alloc(1));
+		GB_CUDA(h, cudaMemsetAsync(h->d_colErr.p, 0, sizeof(PcgGlobal), s));
+	}
+	std::vector<SegCtl> seg(most);
+	for (int c0 = 0; c0 < ncols; c0 += most)
+	{
+		const int k = std::min(most, ncols - c0);
+		GB_CUDA(h, cudaMemcpyAsync(h->d_colB.p, b + (size_t)c0 * n, sizeof(double) * n * k, cudaMemcpyHostToDevice, s));
+		launch_compliance_columns(h->N, k, Wn, h->d_bc.p, h->d_colB.p, true, s);
+		ResArgs a{};
+		d.fill(a, k);
+		h->colLink.fill(a);
+		a.mailStride = mailStride;
+		a.rowStride = rowStride;
+		a.off = h->d_off.p;
+		a.perm = h->d_perm.p;
+		a.maxIter = maxIter;
+		a.tol = h->prm.cg_tolerance;
+		a.timeoutNs = kBarrierTimeoutNs;
+		a.seg = h->d_colSeg.p;
+		a.segStride = 1;
+		a.err = &h->d_colErr.p->err;
+		a.vecStride = n;
+		a.b = h->d_colB.p;
+		a.x = h->d_colX.p;
+		a.val = h->mixed() ? (const void*)h->d_A32.p : h->d_A.p;
+		a.invdiag = h->mixed() ? (const void*)h->d_invdiag32.p : h->d_invdiag.p;
+		a.nrows = h->nrows;
+		GB_CUDA(h, d.launch(a, h->smCount, s));
+		if (Wn) launch_compliance_columns(h->N, k, Wn, nullptr, h->d_colX.p, false, s);
+		GB_CUDA(h, cudaGetLastError());
+		PcgGlobal g;
+		GB_CUDA(h, cudaMemcpyAsync(x + (size_t)c0 * n, h->d_colX.p, sizeof(double) * n * k, cudaMemcpyDeviceToHost, s));
+		GB_CUDA(h, cudaMemcpyAsync(seg.data(), h->d_colSeg.p, sizeof(SegCtl) * k, cudaMemcpyDeviceToHost, s));
+		GB_CUDA(h, cudaMemcpyAsync(&g, h->d_colErr.p, sizeof(PcgGlobal), cudaMemcpyDeviceToHost, s));
+		GB_CUDA(h, cudaStreamSynchronize(s));
+		if (g.err)
+		{
+			GB_CUDA(h, cudaMemsetAsync(h->d_colErr.p, 0, sizeof(PcgGlobal), s));
+			return fail(h, GBFEM_CUDA_ERROR, "compliance CG: a wait for another CTA timed out");
+		}
+		for (int c = 0; c < k; ++c)
+		{
+			// The converging iteration counts here; a column below the threshold from the start has none.
+			const double threshold = std::max(h->prm.cg_tolerance * h->prm.cg_tolerance * seg[c].bb, DBL_MIN);
+			*iterations += seg[c].iter + (seg[c].converged && seg[c].bb >= threshold ? 1 : 0);
+			*allConverged = *allConverged && seg[c].converged;
+		}
+	}
+	return GBFEM_OK;
+}
+
+}  // namespace
+
 gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double* b, double* x, uint32_t flags,
 									int32_t* iterations)
 {
@@ -2131,7 +2344,20 @@ gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double*
 	const Launch L = h->launch();
 	cudaStream_t s = h->stream;
 	const size_t n8 = (size_t)n * kMcgCols;
-	if (!h->d_mcgVec.p)
+	ResDevice* columns = nullptr;
+	if (ncols > 0)
+	{
+		try
+		{
+			const gbfem_status st = compliance_plan(h, ncols, &columns);
+			if (st != GBFEM_OK) return st;
+		}
+		catch (const std::bad_alloc&)
+		{
+			return fail(h, GBFEM_OUT_OF_MEMORY, "gbfem_apply_compliance: out of host memory");
+		}
+	}
+	if (!columns && !h->d_mcgVec.p)
 	{
 		GB_CUDA(h, h->d_mcgVec.alloc(6 * n8));
 		GB_CUDA(h, h->d_mcgPart.alloc(2 * (size_t)kMcgCols * L.vecGrid));
@@ -2158,10 +2384,16 @@ gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double*
 	const MatSellT<float> A32{h->nrows, h->d_perm.p, h->d_off.p, h->d_sellcol.p, h->d_A32.p};
 	const bool m32 = h->mixed();
 	const int maxIter = h->prm.cg_max_iterations > 0 ? h->prm.cg_max_iterations : 2 * n;
-	std::vector<double> hb(n8);
 	int totalIt = 0;
 	bool allConverged = true;
-	for (int c0 = 0; c0 < ncols; c0 += kMcgCols)
+	if (columns)
+	{
+		const gbfem_status st = compliance_resident(h, *columns, ncols, b, x, warp ? h->d_Wn.p : nullptr, maxIter, &totalIt,
+													&allConverged);
+		if (st != GBFEM_OK) return st;
+	}
+	std::vector<double> hb(columns ? 0 : n8);
+	for (int c0 = 0; !columns && c0 < ncols; c0 += kMcgCols)
 	{
 		const int k = std::min(kMcgCols, ncols - c0);
 		std::fill(hb.begin(), hb.end(), 0.0);
@@ -3094,8 +3326,23 @@ struct gbfem_cg_s
 	DevBuf<double> val, invdiag, b, x, r, p, q, part;
 	DevBuf<CgCtl> ctl;
 	CgCtl* h_ctl = nullptr;
+	// Resident solve (gbfem_res.cu, scalar rows): in place of the CSR arrays where its plan fits.
+	ResDevice res;
+	ResExchange link;
+	int smCount = 0, nrows = 0;
+	DevBuf<int> perm, off;
+	DevBuf<double> sell;
+	DevBuf<SegCtl> seg;
+	DevBuf<PcgGlobal> err;
 	void release()
 	{
+		res.free();
+		link.free();
+		perm.free();
+		off.free();
+		sell.free();
+		seg.free();
+		err.free();
 		rowptr.free();
 		col.free();
 		for (auto* d : {&val, &invdiag, &b, &x, &r, &p, &q, &part}) d->free();
@@ -3106,6 +3353,92 @@ struct gbfem_cg_s
 		stream = nullptr;
 	}
 };
+
+namespace {
+
+// Plans the resident solve of a symmetric CSR matrix in the caller's row order (shares are ranges of rows, which in
+// mesh orders couple to a few other ranges) and uploads it; g->res.plan.ok stays false where it does not fit:
+// where the shares' vectors exceed the shared memory, where rows of very different lengths would more than
+// double the matrix in chunks of 32 rows, or where it is eight times the chip's shared memory.
+cudaError_t cg_resident(gbfem_cg g, const std::vector<int>& rowptr, const std::vector<int>& col,
+						const std::vector<double>& val)
+{
+	const int n = g->n, nch = (n + 31) / 32;
+	// Systems of a few unknowns end by exhausting the Krylov space, where one iteration more or less is a
+	// matter of the order of the sums: they keep the order of the row-per-warp product.
+	if (n <= 32) return cudaSuccess;
+	int budget = 0;
+	cudaError_t e = res_budget(g->device, &g->smCount, &budget);
+	if (e != cudaSuccess) return e;
+	std::vector<int> off(nch + 1, 0);
+	int64_t slots = 0;
+	for (int c = 0; c < nch; ++c)
+	{
+		int w = 1;
+		for (int r = 32 * c; r < std::min(n, 32 * c + 32); ++r) w = std::max(w, rowptr[r + 1] - rowptr[r]);
+		slots += w;
+		if (slots * 320 > 8LL * g->smCount * budget) return cudaSuccess;
+		off[c + 1] = (int)slots;
+	}
+	if (slots * 32 > 2LL * rowptr[n] + 4096) return cudaSuccess;
+	const std::vector<int> width = res_widths(kResF64S, 4.0, {slots + 4LL * nch}, {nch}, g->smCount, budget);
+	std::vector<int> rcol(32 * slots), perm(32 * nch);
+	for (int c = 0; c < nch; ++c)
+		for (int l = 0; l < 32; ++l)
+		{
+			const int r = 32 * c + l, k0 = r < n ? rowptr[r] : 0, deg = r < n ? rowptr[r + 1] - k0 : 0;
+			perm[r] = r < n ? r : -1;
+			for (int t = 0; t < off[c + 1] - off[c]; ++t) rcol[(size_t)(off[c] + t) * 32 + l] = t < deg ? col[k0 + t] : r;
+		}
+	ResPlan plan = res_plan(kResF64S, {res_cut(off, 0, nch, width[0])}, off, rcol, {1.0}, g->smCount, budget);
+	if (!plan.ok) return cudaSuccess;
+	std::vector<double> sell(32 * slots, 0.0);
+	for (int r = 0; r < n; ++r)
+		for (int k = rowptr[r]; k < rowptr[r + 1]; ++k)
+			sell[(size_t)(off[r >> 5] + k - rowptr[r]) * 32 + (r & 31)] = val[k];
+	cudaStream_t s = g->stream;
+	g->nrows = 32 * nch;
+	const size_t mailWords = plan.mailWords;
+	e = g->off.upload(off.data(), off.size(), s);
+	if (e == cudaSuccess) e = g->perm.upload(perm.data(), perm.size(), s);
+	if (e == cudaSuccess) e = g->sell.upload(sell.data(), sell.size(), s);
+	if (e == cudaSuccess) e = g->link.reserve(mailWords, (size_t)res_row_words(kResF64S) * g->nrows, s);
+	if (e == cudaSuccess) e = g->seg.alloc(1);
+	if (e == cudaSuccess) e = g->err.alloc(1);
+	if (e == cudaSuccess) e = cudaMemsetAsync(g->err.p, 0, sizeof(PcgGlobal), s);
+	if (e == cudaSuccess) e = g->res.upload(std::move(plan), off, budget, 1, s);
+	return e;
+}
+
+// One resident solve of g->b into g->x; *c: the result.
+gbfem_status cg_solve_resident(gbfem_cg g, int maxIter, SegCtl* c)
+{
+	ResArgs a{};
+	g->res.fill(a, 1);
+	g->link.fill(a);
+	a.off = g->off.p;
+	a.perm = g->perm.p;
+	a.maxIter = maxIter;
+	a.tol = g->tol;
+	a.timeoutNs = kBarrierTimeoutNs;
+	a.seg = g->seg.p;
+	a.err = &g->err.p->err;
+	a.b = g->b.p;
+	a.x = g->x.p;
+	a.val = g->sell.p;
+	a.invdiag = g->invdiag.p;
+	a.nrows = g->nrows;
+	PcgGlobal err;
+	if (g->res.launch(a, g->smCount, g->stream) != cudaSuccess ||
+		cudaMemcpyAsync(c, g->seg.p, sizeof(SegCtl), cudaMemcpyDeviceToHost, g->stream) != cudaSuccess ||
+		cudaMemcpyAsync(&err, g->err.p, sizeof(PcgGlobal), cudaMemcpyDeviceToHost, g->stream) != cudaSuccess ||
+		cudaStreamSynchronize(g->stream) != cudaSuccess)
+		return GBFEM_CUDA_ERROR;
+	if (err.err) cudaMemsetAsync(g->err.p, 0, sizeof(PcgGlobal), g->stream);
+	return err.err ? GBFEM_CUDA_ERROR : GBFEM_OK;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -3148,8 +3481,10 @@ gbfem_status gbfem_cg_create(int32_t n, const int32_t* colptr, const int32_t* ro
 	std::vector<double> valv(ent.size());
 	for (int i = 0; i < n; ++i)
 	{
-		std::sort(ent.begin() + cnt[i], ent.begin() + cnt[i + 1],
-				  [](const std::pair<int, double>& a, const std::pair<int, double>& b) { return a.first < b.first; });
+		// Rows come out sorted where the caller's columns are.
+		auto before = [](const std::pair<int, double>& a, const std::pair<int, double>& b) { return a.first < b.first; };
+		if (!std::is_sorted(ent.begin() + cnt[i], ent.begin() + cnt[i + 1], before))
+			std::sort(ent.begin() + cnt[i], ent.begin() + cnt[i + 1], before);
 		for (int k = cnt[i]; k < cnt[i + 1]; ++k)
 		{
 			colv[k] = ent[k].first;
@@ -3167,11 +3502,19 @@ gbfem_status gbfem_cg_create(int32_t n, const int32_t* colptr, const int32_t* ro
 	};
 	cudaError_t e = cudaSetDevice(device);
 	if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking);
+	if (e == cudaSuccess) e = g->invdiag.upload(invd.data(), n, g->stream);
+	for (auto* d : {&g->b, &g->x})
+		if (e == cudaSuccess) e = d->alloc(n);
+	if (e == cudaSuccess) e = cg_resident(g, cnt, colv, valv);
+	if (e == cudaSuccess && g->res.plan.ok)
+	{
+		*out = g;
+		return GBFEM_OK;
+	}
 	if (e == cudaSuccess) e = g->rowptr.upload(cnt.data(), n + 1, g->stream);
 	if (e == cudaSuccess) e = g->col.upload(colv.data(), colv.size(), g->stream);
 	if (e == cudaSuccess) e = g->val.upload(valv.data(), valv.size(), g->stream);
-	if (e == cudaSuccess) e = g->invdiag.upload(invd.data(), n, g->stream);
-	for (auto* d : {&g->b, &g->x, &g->r, &g->p, &g->q})
+	for (auto* d : {&g->r, &g->p, &g->q})
 		if (e == cudaSuccess) e = d->alloc(n);
 	int grid = std::max(1, std::min((n + 255) / 256, 152 * 8));
 	if (e == cudaSuccess) e = g->part.alloc(partial_slots(grid));
@@ -3209,6 +3552,17 @@ gbfem_status gbfem_cg_solve(gbfem_cg cg, const double* b, double* x, int32_t* it
 	const int maxIter = cg->maxIter > 0 ? cg->maxIter : 2 * cg->n;
 	if (!cuda(cudaMemcpyAsync(cg->b.p, b, sizeof(double) * cg->n, cudaMemcpyHostToDevice, cg->stream)))
 		return GBFEM_CUDA_ERROR;
+	if (cg->res.plan.ok)
+	{
+		SegCtl c;
+		const gbfem_status st = cg_solve_resident(cg, maxIter, &c);
+		if (st != GBFEM_OK || !cuda(cudaMemcpyAsync(x, cg->x.p, sizeof(double) * cg->n, cudaMemcpyDeviceToHost, cg->stream)) ||
+			!cuda(cudaStreamSynchronize(cg->stream)))
+			return GBFEM_CUDA_ERROR;
+		if (iterations) *iterations = c.iter;
+		if (relative_residual) *relative_residual = c.bb > 0 ? std::sqrt(c.rrTrue / c.bb) : 0.0;
+		return c.converged ? GBFEM_OK : GBFEM_CG_MAXITER;
+	}
 	MatCsr A{cg->n, cg->rowptr.p, cg->col.p, cg->val.p};
 	launch_cg_init(cg->n, cg->b.p, cg->invdiag.p, cg->x.p, cg->r.p, cg->p.p, cg->ctl.p, cg->part.p, cg->tol, maxIter, L);
 	long long launched = 0;

@@ -155,6 +155,9 @@ void launch_node_rotation(const DevBody& b, const double* Re, double* Wn, cudaSt
 void launch_prev_positions(int n, const double* x, const double* v, double dt, double* out, cudaStream_t s);
 // X (n x kMcgCols, interleaved) <- blockdiag(W) X, or its transpose.
 void launch_apply_node_rotation(int N, const double* Wn, double* X, bool transpose, cudaStream_t s);
+// The same on ncols columns one after the other (Wn null: no rotation), with zero at the dofs marked in bc (or null).
+void launch_compliance_columns(int N, int ncols, const double* Wn, const uint8_t* bc, double* X, bool transpose,
+							   cudaStream_t s);
 
 // Differentiation form (gbfem_adjoint.cu).
 void launch_element_adjoint(const DevBody& b, const double* x, const double* v, const double* mu, const double* dv,

@@ -969,6 +969,28 @@ __global__ void k_apply_node_rotation(int N, const double* __restrict__ Wn, doub
 	}
 }
 
+// Columns of a node vector one after the other: X <- W X or W^T X per node (Wn null: as it is), and zero at the
+// constrained dofs (bc null: none). Reads and writes each column once.
+__global__ void k_compliance_columns(int N, const double* __restrict__ Wn, const uint8_t* __restrict__ bc,
+									 double* __restrict__ X, int transpose)
+{
+	const int I = blockIdx.x * blockDim.x + threadIdx.x;
+	if (I >= N) return;
+	double* x = X + (size_t)blockIdx.y * 3 * N + 3 * (size_t)I;
+	double v[3] = {x[0], x[1], x[2]};
+	if (Wn)
+	{
+		const double* W = Wn + (size_t)I * 9;
+		const double u[3] = {v[0], v[1], v[2]};
+#pragma unroll
+		for (int i = 0; i < 3; ++i)
+			v[i] = transpose ? (W[i] * u[0] + W[3 + i] * u[1] + W[6 + i] * u[2])
+							 : (W[3 * i] * u[0] + W[3 * i + 1] * u[1] + W[3 * i + 2] * u[2]);
+	}
+#pragma unroll
+	for (int i = 0; i < 3; ++i) x[i] = (bc && bc[3 * I + i]) ? 0.0 : v[i];
+}
+
 __global__ void k_prev_positions(int n, const double* __restrict__ x, const double* __restrict__ v, double dt,
 								 double* __restrict__ out)
 {
@@ -1170,6 +1192,13 @@ void launch_apply_node_rotation(int N, const double* Wn, double* X, bool transpo
 {
 	if (N == 0) return;
 	k_apply_node_rotation<<<blocks((long long)N * C8, 256), 256, 0, s>>>(N, Wn, X, transpose ? 1 : 0);
+}
+
+void launch_compliance_columns(int N, int ncols, const double* Wn, const uint8_t* bc, double* X, bool transpose,
+							   cudaStream_t s)
+{
+	if (N == 0 || ncols == 0) return;
+	k_compliance_columns<<<dim3(blocks(N, 128), ncols), 128, 0, s>>>(N, Wn, bc, X, transpose ? 1 : 0);
 }
 
 void launch_prev_positions(int n, const double* x, const double* v, double dt, double* out, cudaStream_t s)

@@ -23,7 +23,8 @@
 // Solve times, before (gbfem_pcg.cu's, of one launch an iteration or persistent) and here: FP64 80 nodes 2.9
 // and 0.45 ms, 1,331 nodes 3.3 and 0.58, 29,184 nodes 4.1 and 1.33, 24 meshes 10.4 and 3.3; mixed 1,331
 // nodes 1.40 and 0.40, 18,081 nodes 1.93 and 0.53, 270,641 nodes (410 iterations) 18.3 and 15.3, 64 meshes 15.7
-// and 5.7. What bounds them: the two waits of an FP64 iteration (2 x 1.6 us of 5.6) and the one of a mixed
+// and 5.7; 12 compliance columns of 1,331 nodes 47 and 0.94; a caller's matrix of 17,280 rows 2.98 and 0.50.
+// What bounds them: the two waits of an FP64 iteration (2 x 1.6 us of 5.6) and the one of a mixed
 // iteration (1.6 of 4.8), the FP64 rate (64 cycles an instruction of a warp) in FP64 products, and the L2
 // reads of what does not fit in shared memory in large systems.
 
