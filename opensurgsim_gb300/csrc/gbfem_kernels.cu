@@ -9,6 +9,7 @@
 #include <cstdint>
 
 #include "gbfem_element.cuh"
+#include "gbfem_element_fp64.cuh"
 #include "gbfem_internal.h"
 
 namespace gbfem {
@@ -44,6 +45,84 @@ __global__ void __launch_bounds__(kElemThreads) k_element_fp64(DevBody b, const 
 	const int fl = elem::compute<double, kDebug, elem::ElemIn, kLinear>(
 		in, g, lamV, muV, cm, kslots ? kslots + (size_t)e * (kSlots * 9) : nullptr, 1, rhsE + (size_t)e * 12, 1,
 		kDebug ? kfull + (size_t)e * 144 : nullptr, kDebug ? fE + (size_t)e * 12 : nullptr);
+	if (fl & 1) atomicAdd(&counters[1], 1);
+	if (fl & 2) atomicAdd(&counters[0], 1);
+}
+
+// FP64 corotational element kernel of the step: k_element_fp64 without its debug outputs, on compute_fp64's
+// arrangement of the same element. Bound by FP64 issue (64 cycles an instruction of a warp on its scheduler,
+// 19 on the SM): about half the instructions of compute_to, 55 us against 116 at 180 tetrahedra (one warp's
+// instructions one after the other), 0.358 ms against 0.769 at 131,905, 0.60 against 1.31 at 225,000.
+__global__ void __launch_bounds__(kElemThreads) k_element_corot64(DevBody b, const double* __restrict__ xn,
+																  const double* __restrict__ vn,
+																  const double* __restrict__ xt,
+																  const double* __restrict__ vt, double dt, double invDt,
+																  double alpha, double beta, double* __restrict__ kslots,
+																  double* __restrict__ rhsE, int* counters)
+{
+	const int e = blockIdx.x * blockDim.x + threadIdx.x;
+	if (e >= b.E) return;
+	const int E = b.E;
+	// Nodes in ascending order, each with its place in the element.
+	const int4 t4 = b.tets[e];
+	unsigned key[4] = {4u * t4.x, 4u * t4.y + 1u, 4u * t4.z + 2u, 4u * t4.w + 3u};
+	auto order = [&](int i, int j) {
+		const unsigned lo = min(key[i], key[j]), hi = max(key[i], key[j]);
+		key[i] = lo;
+		key[j] = hi;
+	};
+	order(0, 1);
+	order(2, 3);
+	order(0, 2);
+	order(1, 3);
+	order(1, 2);
+	double p[3][3], q[3][3], uK[3][3], uM[4][3], g[3][3];
+	{
+		const bool start = xt == xn && vt == vn;  // uniform: the first Newton iteration
+		double x0[3], r0[3], u0[3];
+#pragma unroll
+		for (int a = 0; a < 4; ++a)
+#pragma unroll
+			for (int k = 0; k < 3; ++k)
+			{
+				const int d = 3 * (int)(key[a] >> 2) + k;
+				const double x = xn[d], v = vn[d], r = b.xrest[d];
+				double u = -(beta + dt) * v, m = -alpha * v;
+				if (!start)
+				{
+					u += x - xt[d];
+					m -= (v - vt[d]) * invDt;
+				}
+				uM[a][k] = m;
+				if (a == 0)
+				{
+					x0[k] = x;
+					r0[k] = r;
+					u0[k] = u;
+					continue;
+				}
+				p[a - 1][k] = x - x0[k];
+				q[a - 1][k] = r - r0[k];
+				uK[a - 1][k] = u - u0[k];
+				g[a - 1][k] = b.rest[(3 * (key[a] & 3u) + k) * (size_t)E + e];
+			}
+	}
+	struct Out
+	{
+		double *ks, *rhs;
+		const unsigned* key;
+		__device__ __forceinline__ bool blocks() const { return ks != nullptr; }
+		__device__ __forceinline__ void rhs_entry(int a, int i, double v) { rhs[3 * (key[a] & 3u) + i] = v; }
+		__device__ __forceinline__ void block(int a, int c, const double (&blk)[9])
+		{
+			const int i = key[a] & 3u, j = key[c] & 3u;
+			double* dst = ks + 9 * (i == j ? i : elem::pair_slot(min(i, j), max(i, j)));
+#pragma unroll
+			for (int k = 0; k < 9; ++k) dst[k] = blk[k];
+		}
+	} out{kslots ? kslots + (size_t)e * (kSlots * 9) : nullptr, rhsE + (size_t)e * 12, key};
+	const int fl = elem::compute_fp64(p, q, uK, uM, g, b.rest[13 * (size_t)E + e], b.rest[14 * (size_t)E + e],
+									  b.rest[15 * (size_t)E + e], b.lumped != 0, out);
 	if (fl & 1) atomicAdd(&counters[1], 1);
 	if (fl & 2) atomicAdd(&counters[0], 1);
 }
@@ -1024,8 +1103,7 @@ void launch_element_fp64(const DevBody& b, const double* xn, const double* vn, c
 		k_element_fp64<false, true><<<nb, kElemThreads, 0, s>>>(b, xn, vn, xt, vt, dt, alpha, beta, kslots, rhsE,
 																 nullptr, nullptr, counters);
 	else
-		k_element_fp64<false, false><<<nb, kElemThreads, 0, s>>>(b, xn, vn, xt, vt, dt, alpha, beta, kslots, rhsE,
-																  nullptr, nullptr, counters);
+		k_element_corot64<<<nb, kElemThreads, 0, s>>>(b, xn, vn, xt, vt, dt, 1.0 / dt, alpha, beta, kslots, rhsE, counters);
 }
 
 int launch_element_f32(const DevBody& b, const double* xn, const double* vn, const double* xt, const double* vt,
