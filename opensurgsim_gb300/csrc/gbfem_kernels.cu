@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kT, 384 / kT) k_element_f32(DevBody b, const d
 	const int cnt = min(kT, E - e0);
 	if (kslots)
 	{
-		// Split layout (k_assemble_f32): the first 8 values of element e's block k as one 32-byte
+		// Split layout (k_assemble): the first 8 values of element e's block k as one 32-byte
 		// sector at kslots[8 (10 e + k)], the 9th at kslots[80 E + 10 e + k].
 		float* dst8 = kslots + (size_t)e0 * (8 * kSlots);
 		for (int idx = threadIdx.x; idx < cnt * 8 * kSlots; idx += kT)
@@ -214,106 +214,100 @@ __global__ void __launch_bounds__(kT, 384 / kT) k_element_f32(DevBody b, const d
 }
 
 // ------------------------------------------------------------------------------------------
-// Assembly: one thread per lower block (I >= J). Sums element blocks in element order, forms
+// Assembly of the lower blocks (I >= J): sums element blocks in element order, forms
 // S = c1 M + c2 K (c1 = 1/dt + alpha, c2 = dt + beta), applies boundary conditions
 // (OdeState.cpp:197-218: zero rows and columns, diagonal 1) and writes the symmetric matrix
 // that Eigen's selfadjointView<Lower> implies into its SELL-32 slots.
+// A block sums up to 24 element blocks, each a dependent pair of loads (index, then values): what bounds both
+// forms is how many of them are under way.
 // ------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void k_assemble(DevBody b, const T* __restrict__ ks, double c1, double c2, T* __restrict__ A,
-						   T* __restrict__ invdiag)
+
+// FP64: one thread an entry, four contributions under way (one thread a block, one under way: 37 us a step of
+// assembly and right-hand side at 180 and at 5,000 tetrahedra, 89 at 131,905; here 17, 19 and 68).
+constexpr int kAsmBlocks = 32;  // lower blocks a CTA
+__global__ void __launch_bounds__(9 * kAsmBlocks) k_assemble(DevBody b, const double* __restrict__ ks, double c1,
+															 double c2, double* __restrict__ A,
+															 double* __restrict__ invdiag)
 {
-	const int L = blockIdx.x * blockDim.x + threadIdx.x;
+	__shared__ double mass[kAsmBlocks];  // one product a block: an FP64 instruction takes 64 cycles of a scheduler
+	const int l0 = blockIdx.x * kAsmBlocks;
+	if (threadIdx.x < kAsmBlocks && l0 + threadIdx.x < b.nl) mass[threadIdx.x] = c1 * b.lmass[l0 + threadIdx.x];
+	__syncthreads();
+	const int l = threadIdx.x / 9, m = threadIdx.x - 9 * l, L = l0 + l;
 	if (L >= b.nl) return;
 	const int4 lb = b.lblk[L];
-	T s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+	const int I = lb.x, J = lb.y, i = m / 3, j = m - 3 * i;
+	const double* from = ks + ((I == J && j > i) ? 3 * j + i : m);  // a diagonal block is read through its lower triangle
+	double s = 0.0;
 	const int k1 = b.cptr[L + 1];
-	for (int k = b.cptr[L]; k < k1; ++k)
+	int k = b.cptr[L];
+	for (; k + 4 <= k1; k += 4)
 	{
-		const T* src = ks + (size_t)b.cidx[k] * 9;
+		double v[4];
 #pragma unroll
-		for (int m = 0; m < 9; ++m) s[m] += src[m];
+		for (int u = 0; u < 4; ++u) v[u] = from[(size_t)b.cidx[k + u] * 9];
+#pragma unroll
+		for (int u = 0; u < 4; ++u) s += v[u];
 	}
-	const T mm = T(c1 * b.lmass[L]);
-	const T c2t = T(c2);
-	T blk[9];
-#pragma unroll
-	for (int m = 0; m < 9; ++m) blk[m] = c2t * s[m];
-	blk[0] += mm;
-	blk[4] += mm;
-	blk[8] += mm;
-	const int I = lb.x, J = lb.y;
-	if (I == J)
-	{
-		blk[1] = blk[3];
-		blk[2] = blk[6];
-		blk[5] = blk[7];
-	}
-#pragma unroll
-	for (int i = 0; i < 3; ++i)
-#pragma unroll
-		for (int j = 0; j < 3; ++j)
-		{
-			const int r = 3 * I + i, c = 3 * J + j;
-			if (b.bc[r] | b.bc[c]) blk[3 * i + j] = (r == c) ? T(1) : T(0);
-		}
-#pragma unroll
-	for (int m = 0; m < 9; ++m) A[(size_t)lb.z + 32 * m] = blk[m];
-	if (lb.w >= 0)
-	{
-#pragma unroll
-		for (int i = 0; i < 3; ++i)
-#pragma unroll
-			for (int j = 0; j < 3; ++j) A[(size_t)lb.w + 32 * (3 * j + i)] = blk[3 * i + j];
-	}
-	if (I == J)
-	{
-#pragma unroll
-		for (int i = 0; i < 3; ++i)
-		{
-			const T d = blk[4 * i];
-			invdiag[3 * I + i] = (d != T(0)) ? T(1) / d : T(1);  // DiagonalPreconditioner
-		}
-	}
+	for (; k < k1; ++k) s += from[(size_t)b.cidx[k] * 9];
+	double v = i == j ? fma(c2, s, mass[l]) : c2 * s;
+	const int r = 3 * I + i, c = 3 * J + j;
+	if (b.bc[r] | b.bc[c]) v = (r == c) ? 1.0 : 0.0;
+	A[(size_t)lb.z + 32 * m] = v;
+	if (lb.w >= 0) A[(size_t)lb.w + 32 * (3 * j + i)] = v;
+	if (r == c) invdiag[r] = (v != 0.0) ? 1.0 / v : 1.0;  // DiagonalPreconditioner
 }
 
-// FP32 assembly from the FP32 element kernel's split layout: each contribution's first 8 values are
-// one aligned 32-byte sector (two float4 loads), the 9th sits in the trailing array. The 36-byte blocks
-// of the plain layout straddle sectors, so a contribution cost two sectors of reads there. Same sums,
-// same order as k_assemble.
-__global__ void k_assemble_f32(DevBody b, const float* __restrict__ ks, double c1, double c2, float* __restrict__ A,
-							   float* __restrict__ invdiag)
+// FP32, from the element kernel's split layout: a contribution's first 8 values are one aligned 32-byte sector
+// (two float4 loads), the 9th sits in the trailing array (the 36-byte blocks of the plain layout straddle
+// sectors, two of reads each). One thread a block, four contributions under way: 0.207 ms for assembly
+// and right-hand side of the 1.28M-tetrahedron bar and 0.393 of a batch of 3.2M, against 0.266 and
+// 0.502 with one under way (0.220 and 0.413 with two; one thread an entry as above: 0.297 and 0.625).
+__global__ void __launch_bounds__(128) k_assemble_f32(DevBody b, const float* __restrict__ ks, double c1, double c2,
+													  float* __restrict__ A, float* __restrict__ invdiag)
 {
 	const int L = blockIdx.x * blockDim.x + threadIdx.x;
 	if (L >= b.nl) return;
+	constexpr int kIn = 4;
 	const int4 lb = b.lblk[L];
 	float s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 	const float* ks1 = ks + (size_t)b.E * (8 * kSlots);
 	const int k1 = b.cptr[L + 1];
-	for (int k = b.cptr[L]; k < k1; ++k)
+	int k = b.cptr[L];
+	for (; k < k1; k += kIn)
 	{
-		const int ci = b.cidx[k];
-		const float4* src = reinterpret_cast<const float4*>(ks + (size_t)ci * 8);
-		const float4 u = src[0], w = src[1];
-		const float t = ks1[ci];
-		s[0] += u.x;
-		s[1] += u.y;
-		s[2] += u.z;
-		s[3] += u.w;
-		s[4] += w.x;
-		s[5] += w.y;
-		s[6] += w.z;
-		s[7] += w.w;
-		s[8] += t;
+		float4 u[kIn], w[kIn];
+		float t[kIn];
+#pragma unroll
+		for (int q = 0; q < kIn; ++q)
+			if (k + q < k1)
+			{
+				const int ci = b.cidx[k + q];
+				const float4* src = reinterpret_cast<const float4*>(ks + (size_t)ci * 8);
+				u[q] = src[0];
+				w[q] = src[1];
+				t[q] = ks1[ci];
+			}
+#pragma unroll
+		for (int q = 0; q < kIn; ++q)
+			if (k + q < k1)
+			{
+				s[0] += u[q].x;
+				s[1] += u[q].y;
+				s[2] += u[q].z;
+				s[3] += u[q].w;
+				s[4] += w[q].x;
+				s[5] += w[q].y;
+				s[6] += w[q].z;
+				s[7] += w[q].w;
+				s[8] += t[q];
+			}
 	}
 	const float mm = float(c1 * b.lmass[L]);
 	const float c2t = float(c2);
 	float blk[9];
 #pragma unroll
-	for (int m = 0; m < 9; ++m) blk[m] = c2t * s[m];
-	blk[0] += mm;
-	blk[4] += mm;
-	blk[8] += mm;
+	for (int m = 0; m < 9; ++m) blk[m] = m % 4 == 0 ? fma(c2t, s[m], mm) : c2t * s[m];
 	const int I = lb.x, J = lb.y;
 	if (I == J)
 	{
@@ -349,64 +343,48 @@ __global__ void k_assemble_f32(DevBody b, const float* __restrict__ ks, double c
 	}
 }
 
+// Right-hand side of a dof: its node's element shares in element order, four under way at a time.
 template <typename T>
 __global__ void k_rhs_gather(DevBody b, const T* __restrict__ rhsE, double g0, double g1, double g2, int gravityOn,
 							 double* __restrict__ rhs, int applyBc)
 {
-	const int I = blockIdx.x * blockDim.x + threadIdx.x;
-	if (I >= b.N) return;
-	double s0 = 0, s1 = 0, s2 = 0;
+	const int d = blockIdx.x * blockDim.x + threadIdx.x;
+	if (d >= 3 * b.N) return;
+	const int I = d / 3, i = d - 3 * I;
 	const int k1 = b.iptr[I + 1];
-	if constexpr (std::is_same<T, float>::value)
-	{
-		// FP32 contributions summed exactly enough as float pairs (TwoSum; the errors' own sum keeps
-		// ~2^-48 of the total) and converted to FP64 once: an FP64 add and conversion per contribution
-		// (~140 FP64 instructions a node) would issue at 1/64 of the FP32 rate.
-		float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
-		for (int k = b.iptr[I]; k < k1; ++k)
+	int k = b.iptr[I];
+	double s = 0.0;
+	// FP32 contributions are summed exactly enough as float pairs (TwoSum; the errors' own sum keeps
+	// ~2^-48 of the total) and converted to FP64 once: an FP64 add and conversion per contribution
+	// would issue at 1/64 of the FP32 rate.
+	float h = 0.f, lo = 0.f;
+	auto add = [&](T v) {
+		if constexpr (std::is_same<T, float>::value)
 		{
-			const int c = b.iidx[k];
-			const float* src = rhsE + (size_t)(c >> 2) * 12 + 3 * (c & 3);
+			float t, e;
+			elem::df_two_sum(h, v, t, e);
+			h = t;
+			lo = __fadd_rn(lo, e);
+		}
+		else
+			s += v;
+	};
+	auto at = [&](int q) {
+		const int c = b.iidx[q];
+		return rhsE[(size_t)(c >> 2) * 12 + 3 * (c & 3) + i];
+	};
+	for (; k + 4 <= k1; k += 4)
+	{
+		T v[4];
 #pragma unroll
-			for (int i = 0; i < 3; ++i)
-			{
-				float t, e;
-				elem::df_two_sum(h[i], src[i], t, e);
-				h[i] = t;
-				l[i] = __fadd_rn(l[i], e);
-			}
-		}
-		s0 = double(h[0]) + double(l[0]);
-		s1 = double(h[1]) + double(l[1]);
-		s2 = double(h[2]) + double(l[2]);
+		for (int u = 0; u < 4; ++u) v[u] = at(k + u);
+#pragma unroll
+		for (int u = 0; u < 4; ++u) add(v[u]);
 	}
-	else
-	{
-		for (int k = b.iptr[I]; k < k1; ++k)
-		{
-			const int c = b.iidx[k];
-			const T* src = rhsE + (size_t)(c >> 2) * 12 + 3 * (c & 3);
-			s0 += double(src[0]);
-			s1 += double(src[1]);
-			s2 += double(src[2]);
-		}
-	}
-	if (gravityOn)  // FemRepresentation::addGravityForce (:641-662)
-	{
-		const double m = b.nmass[I];
-		s0 += g0 * m;
-		s1 += g1 * m;
-		s2 += g2 * m;
-	}
-	if (applyBc)
-	{
-		if (b.bc[3 * I]) s0 = 0.0;
-		if (b.bc[3 * I + 1]) s1 = 0.0;
-		if (b.bc[3 * I + 2]) s2 = 0.0;
-	}
-	rhs[3 * I] = s0;
-	rhs[3 * I + 1] = s1;
-	rhs[3 * I + 2] = s2;
+	for (; k < k1; ++k) add(at(k));
+	if constexpr (std::is_same<T, float>::value) s = double(h) + double(lo);
+	if (gravityOn) s += (i == 0 ? g0 : (i == 1 ? g1 : g2)) * b.nmass[I];  // FemRepresentation::addGravityForce (:641-662)
+	rhs[d] = (applyBc && b.bc[d]) ? 0.0 : s;
 }
 
 __global__ void k_assemble_full_csc(int nnz, const int* __restrict__ sptr, const int* __restrict__ sidx,
@@ -1141,7 +1119,7 @@ void launch_assemble(const DevBody& b, const double* kslots, double c1, double c
 					 cudaStream_t s)
 {
 	if (b.nl == 0) return;
-	k_assemble<double><<<blocks(b.nl, 128), 128, 0, s>>>(b, kslots, c1, c2, A, invdiag);
+	k_assemble<<<blocks(b.nl, kAsmBlocks), 9 * kAsmBlocks, 0, s>>>(b, kslots, c1, c2, A, invdiag);
 }
 
 void launch_assemble(const DevBody& b, const float* kslots, double c1, double c2, float* A, float* invdiag,
@@ -1155,7 +1133,7 @@ void launch_rhs_gather(const DevBody& b, const double* rhsE, const double* gravi
 					   int applyBc, cudaStream_t s)
 {
 	if (b.N == 0) return;
-	k_rhs_gather<double><<<blocks(b.N, 128), 128, 0, s>>>(b, rhsE, gravity[0], gravity[1], gravity[2], gravityOn, rhs,
+	k_rhs_gather<double><<<blocks(3LL * b.N, 192), 192, 0, s>>>(b, rhsE, gravity[0], gravity[1], gravity[2], gravityOn, rhs,
 														  applyBc);
 }
 
@@ -1163,7 +1141,7 @@ void launch_rhs_gather(const DevBody& b, const float* rhsE, const double* gravit
 					   int applyBc, cudaStream_t s)
 {
 	if (b.N == 0) return;
-	k_rhs_gather<float><<<blocks(b.N, 128), 128, 0, s>>>(b, rhsE, gravity[0], gravity[1], gravity[2], gravityOn, rhs,
+	k_rhs_gather<float><<<blocks(3LL * b.N, 192), 192, 0, s>>>(b, rhsE, gravity[0], gravity[1], gravity[2], gravityOn, rhs,
 														 applyBc);
 }
 
