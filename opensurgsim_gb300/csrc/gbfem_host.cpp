@@ -313,6 +313,7 @@ struct gbfem_handle_s
 	ResDevice d_res;
 	ResExchange resLink;
 	int resBudget = 0;
+	float resNear = 1.f;  // ResArgs::nearFraction
 	int resForm() const { return res.ok ? res.form : (mixed() ? kResMixed : kResF64); }
 	DevBuf<float4> d_resOwn;  // kResMixedFar: p and x_delta of every row
 	// Compliance columns: plans by CTAs a column, their exchange, columns and results.
@@ -742,6 +743,21 @@ gbfem_status upload_resident(gbfem_handle h, const std::vector<int>& off)
 	GB_CUDA(h, h->resLink.reserve(h->res.mailWords, (size_t)res_row_words(form) * h->nrows, h->stream));
 	if (form == kResMixedFar) GB_CUDA(h, h->d_resOwn.alloc(2 * (size_t)h->nrows));
 	GB_CUDA(h, h->d_res.upload(ResPlan(h->res), off, h->resBudget, 1, h->stream));
+	if (h->mixed() && !h->batched())
+	{
+		// A system that streams more than L2 (129 MB) holds beside the other vectors keeps 75 MB of it there, less as
+		// the stream's own lines need more room. Solves at 1, 0.8, 0.6, 0.4, 0.2 of the stream kept: 94 MB 1.67, 1.58,
+		// 1.68, 1.77, 1.85 ms; 116 MB 2.53, 2.35, 2.15, 2.19, 2.26; 148 MB 3.35, 3.35, 3.19, 2.84, 2.81; 269 MB 4.48,
+		// 4.57, 4.57, 4.57, 4.21 and 4.07 at 0.1; up to 76 MB all of it is best. The systems of a batch take turns
+		// and find theirs there.
+		double mb = 0.0;
+		for (const ResPart& p : h->res.parts)
+		{
+			const ResLayout L = res_layout(form, p.c1 - p.c0, p.h1 - p.h0);
+			mb += std::max(0.0, 1e-6 * ((double)(off[p.c1] - off[p.c0]) * L.slotBytes - ((int)h->d_res.smem - L.mat)));
+		}
+		h->resNear = (float)std::min(1.0, std::max(0.02, (75.0 - 0.4 * std::max(0.0, mb - 120.0)) / std::max(mb, 1.0)));
+	}
 	std::vector<uint16_t>().swap(h->res.lcol);
 	return GBFEM_OK;
 }
@@ -1349,6 +1365,7 @@ gbfem_status enqueue_resident(gbfem_handle h, const double* b, double* x, int ma
 	a.segMaxIter = segCaps ? h->d_segMaxIter.p : nullptr;
 	a.tol = h->prm.cg_tolerance;
 	a.drop = kRefreshDrop;
+	a.nearFraction = h->resNear;
 	a.timeoutNs = kBarrierTimeoutNs;
 	a.seg = h->d_seg.p;
 	a.err = &h->d_pcgGlobal.p->err;

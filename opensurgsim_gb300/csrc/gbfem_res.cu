@@ -361,33 +361,20 @@ struct AccMul
 	template <bool kGlobal>
 	__device__ __forceinline__ void run(const M* v, const uint16_t* col, int s, int e)
 	{
-		constexpr int U = 2;  // slots in flight
-#pragma unroll 1
-		for (; s < e; s += U)
+#pragma unroll 2
+		for (; s < e; ++s)
 		{
-			int J[U];
-			M m[U][bs * bs];
+			const int J = kGlobal ? (int)__ldg(&col[(size_t)s * 32]) : (int)col[s * 32];
+			M m[bs * bs];
 #pragma unroll
-			for (int k = 0; k < U; ++k)
-				if (s + k < e)
-				{
-					J[k] = kGlobal ? (int)__ldg(&col[(size_t)(s + k) * 32]) : (int)col[(s + k) * 32];
+			for (int j = 0; j < bs * bs; ++j) m[j] = kGlobal ? __ldg(&v[(size_t)s * kVal + 32 * j]) : v[s * kVal + 32 * j];
+			V x[bs];
 #pragma unroll
-					for (int j = 0; j < bs * bs; ++j)
-						m[k][j] = kGlobal ? __ldg(&v[(size_t)(s + k) * kVal + 32 * j]) : v[(s + k) * kVal + 32 * j];
-				}
+			for (int j = 0; j < bs; ++j) x[j] = shm<V>(u)[bs * J + j];
 #pragma unroll
-			for (int k = 0; k < U; ++k)
-				if (s + k < e)
-				{
-					V x[bs];
+			for (int i = 0; i < bs; ++i)
 #pragma unroll
-					for (int j = 0; j < bs; ++j) x[j] = shm<V>(u)[bs * J[k] + j];
-#pragma unroll
-					for (int i = 0; i < bs; ++i)
-#pragma unroll
-						for (int j = 0; j < bs; ++j) y[i] = fma(V(m[k][i * bs + j]), x[j], y[i]);
-				}
+				for (int j = 0; j < bs; ++j) y[i] = fma(V(m[i * bs + j]), x[j], y[i]);
 		}
 	}
 	__device__ __forceinline__ void put(int base, int at)
@@ -797,6 +784,7 @@ struct MixedShare
 	ResLayout L;
 	int c0, nHalo, first, last;  // this warp's entries of the chunk list
 	int colKept;                 // shared offset of the kept columns
+	unsigned long long policy;   // L2 policy of the slots read in every product
 	const float* val;            // the share's first slot
 	const uint16_t* col;
 };
@@ -820,6 +808,7 @@ __device__ __forceinline__ MixedShare open_mixed(const ResArgs& a, const ResPart
 	S.val = static_cast<const float*>(a.val) + (size_t)k0 * 288;
 	S.col = a.lcol + (size_t)k0 * 32;
 	S.colKept = S.L.mat + kept * 1152;
+	asm("createpolicy.fractional.L2::evict_normal.L2::evict_first.b64 %0, %1;" : "=l"(S.policy) : "f"(a.nearFraction));
 	int* offL = shm<int>(S.L.offL);
 	int* keptL = shm<int>(S.L.pieces);  // first kept slot of a chunk: an even share of every chunk's slots
 	int* halo = shm<int>(S.L.halo);
@@ -847,46 +836,77 @@ __device__ __forceinline__ MixedShare open_mixed(const ResArgs& a, const ResPart
 	return S;
 }
 
-// Calls f(values, columns, n) for the kept and then the other slots of chunk c (this lane's row).
+// Loads of matrix words that no one else reads, with the share's L2 policy: where the matrix does not fit in L2, a
+// part of its lines stays and the others leave first, so that part is found there in every product (all of them
+// in turn would push one another out; ResArgs::nearFraction).
+__device__ __forceinline__ float ld_hint(const float* p, unsigned long long policy)
+{
+	float v;
+	asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
+	return v;
+}
+__device__ __forceinline__ int ld_hint(const uint16_t* p, unsigned long long policy)
+{
+	unsigned short v;
+	asm("ld.global.nc.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(policy));
+	return v;
+}
+
+// A chunk's kept slots.
+struct KeptSlots
+{
+	int val, col;  // shared offsets of this lane's values and columns
+	__device__ __forceinline__ int column(int k) const { return shm<uint16_t>(col)[32 * k]; }
+	__device__ __forceinline__ void values(int k, float (&m)[9]) const
+	{
+#pragma unroll
+		for (int j = 0; j < 9; ++j) m[j] = shm<float>(val)[288 * k + 32 * j];
+	}
+};
+// A chunk's other slots, in global memory.
+struct FarSlots
+{
+	const float* val;
+	const uint16_t* col;
+	unsigned long long policy;
+	__device__ __forceinline__ int column(int k) const { return ld_hint(&col[32 * k], policy); }
+	__device__ __forceinline__ void values(int k, float (&m)[9]) const
+	{
+#pragma unroll
+		for (int j = 0; j < 9; ++j) m[j] = ld_hint(&val[288 * k + 32 * j], policy);
+	}
+};
+
+// Calls f(slots, n) for the kept and then the other slots of chunk c (this lane's row).
 template <typename F>
 __device__ __forceinline__ void chunk_slots(const MixedShare& S, int c, F f)
 {
 	const int lane = threadIdx.x & 31;
 	const int o = shm<int>(S.L.offL)[c], o1 = shm<int>(S.L.offL)[c + 1];
 	const int d = shm<int>(S.L.pieces)[c], n = shm<int>(S.L.pieces)[c + 1] - d;
-	f(std::false_type(), shm<float>(S.L.mat) + d * 288 + lane, shm<uint16_t>(S.colKept) + d * 32 + lane, n);
-	if (n < o1 - o) f(std::true_type(), S.val + (size_t)(o + n) * 288 + lane, S.col + (size_t)(o + n) * 32 + lane, o1 - o - n);
+	f(KeptSlots{S.L.mat + d * 1152 + 4 * lane, S.colKept + d * 64 + 2 * lane}, n);
+	if (n < o1 - o)
+		f(FarSlots{S.val + (size_t)(o + n) * 288 + lane, S.col + (size_t)(o + n) * 32 + lane, S.policy}, o1 - o - n);
 }
 
 // w = A u for the rows of chunk c, slot by slot with the roundings of k_pcg_persistent's products.
 __device__ __forceinline__ void multiply(const MixedShare& S, const float4* U, int c, float& a0, float& a1, float& a2)
 {
-	chunk_slots(S, c, [&](auto global, const float* v, const uint16_t* col, int n) {
-		constexpr bool kGlobal = decltype(global)::value;
-		constexpr int kIn = kGlobal ? 2 : 4;  // slots in flight (four global ones spill)
-#pragma unroll 1
-		for (int k = 0; k < n; k += kIn)
+	chunk_slots(S, c, [&](const auto& slots, int n) {
+		// A plain loop: rounds of guarded loads took twice as long in shared memory (19 slots: 2,680 cycles of a
+		// warp, here 1,410; 15 warps at once are bound by the shared-memory pipe's 14 words a slot).
+		constexpr bool kFar = std::is_same<std::decay_t<decltype(slots)>, FarSlots>::value;
+		constexpr int kUnroll = kFar ? 2 : 6;  // far slots: 12.0 ms a solve of 270,641 nodes at 2, 12.7 at 3, 12.4 at 4
+#pragma unroll kUnroll
+		for (int k = 0; k < n; ++k)
 		{
-			int J[kIn];
-			float m[kIn][9];
-#pragma unroll
-			for (int i = 0; i < kIn; ++i)
-				if (k + i < n)
-				{
-					J[i] = kGlobal ? (int)__ldg(&col[(k + i) * 32]) : (int)col[(k + i) * 32];
-#pragma unroll
-					for (int j = 0; j < 9; ++j)
-						m[i][j] = kGlobal ? __ldg(&v[(k + i) * 288 + 32 * j]) : v[(k + i) * 288 + 32 * j];
-				}
-#pragma unroll
-			for (int i = 0; i < kIn; ++i)
-				if (k + i < n)
-				{
-					const float4 u = U[J[i]];
-					a0 += m[i][0] * u.x + m[i][1] * u.y + m[i][2] * u.z;
-					a1 += m[i][3] * u.x + m[i][4] * u.y + m[i][5] * u.z;
-					a2 += m[i][6] * u.x + m[i][7] * u.y + m[i][8] * u.z;
-				}
+			float m[9];
+			const int J = slots.column(k);
+			slots.values(k, m);
+			const float4 u = U[J];
+			a0 += m[0] * u.x + m[1] * u.y + m[2] * u.z;
+			a1 += m[3] * u.x + m[4] * u.y + m[5] * u.z;
+			a2 += m[6] * u.x + m[7] * u.y + m[8] * u.z;
 		}
 	});
 }
@@ -999,24 +1019,24 @@ __device__ __forceinline__ void rows_mixed(const ResArgs& a, const ResPart p, un
 			{
 				const int c = a.chunkList[j], i = 32 * c + lane;
 				float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
-				chunk_slots(S, c, [&](auto global, const float* v, const uint16_t* col, int n) {
-					constexpr bool kGlobal = decltype(global)::value;
-#pragma unroll 1
-					for (int k = 0; k < n; ++k, v += 288, col += 32)
+				chunk_slots(S, c, [&](const auto& slots, int n) {
+#pragma unroll 2
+					for (int k = 0; k < n; ++k)
 					{
-						const int J = kGlobal ? (int)__ldg(col) : (int)*col;
+						const int J = slots.column(k);
+						float v[9];
+						slots.values(k, v);
 						const float4 tv = U[J], lv = R[J];
 						const float x[3] = {tv.x, tv.y, tv.z}, y[3] = {lv.x, lv.y, lv.z};
 #pragma unroll
 						for (int m = 0; m < 9; ++m)
 						{
-							const float av = kGlobal ? __ldg(&v[32 * m]) : v[32 * m];
-							const float q = __fmul_rn(av, x[m % 3]);
-							const float qe = __fmaf_rn(av, x[m % 3], -q);
+							const float q = __fmul_rn(v[m], x[m % 3]);
+							const float qe = __fmaf_rn(v[m], x[m % 3], -q);
 							float hs, he;
 							two_sum(hi[m / 3], q, hs, he);
 							hi[m / 3] = hs;
-							lo[m / 3] = __fadd_rn(lo[m / 3], __fadd_rn(he, __fmaf_rn(av, y[m % 3], qe)));
+							lo[m / 3] = __fadd_rn(lo[m / 3], __fadd_rn(he, __fmaf_rn(v[m], y[m % 3], qe)));
 						}
 #pragma unroll
 						for (int m = 0; m < 3; ++m)
@@ -1061,35 +1081,48 @@ __device__ __forceinline__ void rows_mixed(const ResArgs& a, const ResPart p, un
 		{
 			// p = u + beta p, s = w + beta s, x += alpha p, r -= alpha s, u = d r.
 			const float al = sh.al, be = sh.be, as = sh.as;
-#pragma unroll 1
-			for (int i = tid; i < nLoc; i += kRowThreads)
+			struct Row
 			{
-				float4 u = U[i], r = R[i], s = Sv[i];
-				const float4 w = W[i];
+				float4 u, r, s, w, q, x;
+			};
+			auto load = [&](int i, Row& v) {
+				v.u = U[i], v.r = R[i], v.s = Sv[i], v.w = W[i];
+				if (i < nOwn) v.q = P[i], v.x = X[i];
+			};
+			auto advance = [&](int i, Row& v) {
 				if (i < nOwn)
 				{
-					float4 q = P[i], x = X[i];
-					q.x = __fmaf_rn(be, q.x, u.x);
-					q.y = __fmaf_rn(be, q.y, u.y);
-					q.z = __fmaf_rn(be, q.z, u.z);
-					x.x = __fmaf_rn(as, q.x, x.x);
-					x.y = __fmaf_rn(as, q.y, x.y);
-					x.z = __fmaf_rn(as, q.z, x.z);
-					P[i] = q;
-					X[i] = x;
+					v.q.x = __fmaf_rn(be, v.q.x, v.u.x);
+					v.q.y = __fmaf_rn(be, v.q.y, v.u.y);
+					v.q.z = __fmaf_rn(be, v.q.z, v.u.z);
+					v.x.x = __fmaf_rn(as, v.q.x, v.x.x);
+					v.x.y = __fmaf_rn(as, v.q.y, v.x.y);
+					v.x.z = __fmaf_rn(as, v.q.z, v.x.z);
+					P[i] = v.q;
+					X[i] = v.x;
 				}
-				s.x = __fmaf_rn(be, s.x, w.x);
-				s.y = __fmaf_rn(be, s.y, w.y);
-				s.z = __fmaf_rn(be, s.z, w.z);
-				r.x = __fmaf_rn(-al, s.x, r.x);
-				r.y = __fmaf_rn(-al, s.y, r.y);
-				r.z = __fmaf_rn(-al, s.z, r.z);
-				u.x = __fmul_rn(u.w, r.x);
-				u.y = __fmul_rn(r.w, r.y);
-				u.z = __fmul_rn(s.w, r.z);
-				Sv[i] = s;
-				R[i] = r;
-				U[i] = u;
+				v.s.x = __fmaf_rn(be, v.s.x, v.w.x);
+				v.s.y = __fmaf_rn(be, v.s.y, v.w.y);
+				v.s.z = __fmaf_rn(be, v.s.z, v.w.z);
+				v.r.x = __fmaf_rn(-al, v.s.x, v.r.x);
+				v.r.y = __fmaf_rn(-al, v.s.y, v.r.y);
+				v.r.z = __fmaf_rn(-al, v.s.z, v.r.z);
+				v.u.x = __fmul_rn(v.u.w, v.r.x);
+				v.u.y = __fmul_rn(v.r.w, v.r.y);
+				v.u.z = __fmul_rn(v.s.w, v.r.z);
+				Sv[i] = v.s;
+				R[i] = v.r;
+				U[i] = v.u;
+			};
+#pragma unroll 1
+			for (int i = tid; i < nLoc; i += 2 * kRowThreads)
+			{
+				const int i2 = i + kRowThreads;
+				Row v, v2;
+				load(i, v);
+				if (i2 < nLoc) load(i2, v2);
+				advance(i, v);
+				if (i2 < nLoc) advance(i2, v2);
 			}
 		}
 		else
@@ -1179,6 +1212,8 @@ __device__ __forceinline__ void rows_mixed(const ResArgs& a, const ResPart p, un
 #pragma unroll
 			for (int k = 0; k < 3; ++k) sh.red[k][warp] = make_float2(sum[k].h, sum[k].l);
 		sums_ready();
+		// Warps without a chunk left wait here for the others: their polls would take the shared-memory pipe from them.
+		rows_sync();
 		fetch_halo<1>(a, S, words, tag, [&](int i, const ResWord(&v)[1]) { put_xyz(W[i], v[0]); });
 		scalars_wait();
 	}

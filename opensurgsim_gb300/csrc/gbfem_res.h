@@ -53,6 +53,7 @@ struct ResArgs
 	const int* perm;      // row position -> node (or scalar row), -1 on padding rows
 	const int* segMaxIter;  // per system, or null: maxIter
 	int maxIter, smemBudget;
+	float nearFraction;   // mixed forms: part of the slots beyond shared memory that L2 is to keep
 	double tol, drop;
 	long long timeoutNs;
 	ResWord* mail;        // mailboxes of all systems; right-hand side c uses mail + c * mailStride
