@@ -756,7 +756,8 @@ gbfem_status upload_resident(gbfem_handle h, const std::vector<int>& off)
 			const ResLayout L = res_layout(form, p.c1 - p.c0, p.h1 - p.h0);
 			mb += std::max(0.0, 1e-6 * ((double)(off[p.c1] - off[p.c0]) * L.slotBytes - ((int)h->d_res.smem - L.mat)));
 		}
-		h->resNear = (float)std::min(1.0, std::max(0.02, (75.0 - 0.4 * std::max(0.0, mb - 120.0)) / std::max(mb, 1.0)));
+		const double keep = std::min(75.0, std::max(75.0 - 0.9 * (mb - 120.0), 90.0 - 0.3 * mb));
+		h->resNear = (float)std::min(1.0, std::max(0.02, keep / std::max(mb, 1.0)));
 	}
 	std::vector<uint16_t>().swap(h->res.lcol);
 	return GBFEM_OK;

@@ -386,73 +386,75 @@ struct AccMul
 	__device__ __forceinline__ void cut(int piece) { put(part, piece * 32 + (threadIdx.x & 31)); }
 };
 
-// Row warps: waits for NW words of every halo row (word k of row rs at rows[k * nrows + rs]) and stores them
-// by put(local row, words). Two rows a thread are in flight at once.
+// Waits for N words with this tag, given by their addresses.
+template <int N>
+__device__ __forceinline__ void wait_words(const ResArgs& a, const ResWord* const (&p)[N], unsigned tag, ResWord (&w)[N])
+{
+	Patience wait;
+	for (;;)
+	{
+		bool all = true;
+#pragma unroll
+		for (int k = 0; k < N; ++k) w[k] = ld_word(p[k]);
+#pragma unroll
+		for (int k = 0; k < N; ++k) all = all && w[k].tag == tag;
+		if (all) break;
+		if (wait.lost(a))
+		{
+			sh.bad = 1;
+			break;
+		}
+	}
+}
+
+// Row warps: waits for `words` of every halo element (n of them, word e at words[at(e)]) and stores them by
+// put(e, word); two elements a thread are in flight while there are two.
+template <int NW, typename A, typename F>
+__device__ __forceinline__ void fetch(const ResArgs& a, int n, const ResWord* words, unsigned tag, A at, F put)
+{
+	int j = threadIdx.x;
+#pragma unroll 1
+	for (; j + kRowThreads < n; j += 2 * kRowThreads)
+	{
+		const ResWord *q = words + at(j), *q2 = words + at(j + kRowThreads), *p[2 * NW];
+		ResWord w[2 * NW], u[NW];
+#pragma unroll
+		for (int k = 0; k < NW; ++k) p[k] = q + (size_t)k * a.nrows, p[NW + k] = q2 + (size_t)k * a.nrows;
+		wait_words(a, p, tag, w);
+#pragma unroll
+		for (int k = 0; k < NW; ++k) u[k] = w[k];
+		put(j, u);
+#pragma unroll
+		for (int k = 0; k < NW; ++k) u[k] = w[NW + k];
+		put(j + kRowThreads, u);
+	}
+	if (j < n)
+	{
+		const ResWord *q = words + at(j), *p[NW];
+		ResWord u[NW];
+#pragma unroll
+		for (int k = 0; k < NW; ++k) p[k] = q + (size_t)k * a.nrows;
+		wait_words(a, p, tag, u);
+		put(j, u);
+	}
+}
+
+// The halo rows of a share, NW words a row (word k of row rs at rows[k * nrows + rs]): put(local row, words).
 template <int NW, typename S_, typename F>
 __device__ __forceinline__ void fetch_halo(const ResArgs& a, const S_& S, const ResWord* rows, unsigned tag, F put)
 {
 	const int* halo = shm<int>(S.L.halo);
-	for (int j = threadIdx.x; j < S.nHalo; j += 2 * kRowThreads)
-	{
-		const int j2 = j + kRowThreads;
-		const bool two = j2 < S.nHalo;
-		const ResWord* p = rows + halo[j];
-		const ResWord* q = rows + halo[two ? j2 : j];
-		ResWord w[NW], w2[NW];
-		Patience wait;
-		for (;;)
-		{
-			bool all = true;
-#pragma unroll
-			for (int k = 0; k < NW; ++k)
-			{
-				w[k] = ld_word(p + (size_t)k * a.nrows);
-				if (two) w2[k] = ld_word(q + (size_t)k * a.nrows);
-			}
-#pragma unroll
-			for (int k = 0; k < NW; ++k) all = all && w[k].tag == tag && (!two || w2[k].tag == tag);
-			if (all) break;
-			if (wait.lost(a))
-			{
-				sh.bad = 1;
-				break;
-			}
-		}
-		put(S.L.nOwn + j, w);
-		if (two) put(S.L.nOwn + j2, w2);
-	}
+	fetch<NW>(a, S.nHalo, rows, tag, [&](int j) { return halo[j]; },
+			  [&](int j, const ResWord(&w)[NW]) { put(S.L.nOwn + j, w); });
 }
 
-// Row warps: waits for every word of the halo rows, bs words a row, and stores them by put(local element,
-// word). Two words a thread are in flight at once.
+// The halo rows of a share element by element, bs words a row: put(local element, word).
 template <int bs, typename F>
 __device__ __forceinline__ void fetch_words(const ResArgs& a, const Share& S, const ResWord* words, unsigned tag, F put)
 {
 	const int* halo = shm<int>(S.L.halo);
-	const int n = bs * S.nHalo, own = bs * S.L.nOwn;
-#pragma unroll 1
-	for (int j = threadIdx.x; j < n; j += 2 * kRowThreads)
-	{
-		const int j2 = j + kRowThreads;
-		const bool two = j2 < n;
-		const ResWord* p = words + (bs * halo[j / bs] + j % bs);
-		const ResWord* q = two ? words + (bs * halo[j2 / bs] + j2 % bs) : p;
-		ResWord w, w2;
-		Patience wait;
-		for (;;)
-		{
-			w = ld_word(p);
-			w2 = ld_word(q);
-			if (w.tag == tag && w2.tag == tag) break;
-			if (wait.lost(a))
-			{
-				sh.bad = 1;
-				break;
-			}
-		}
-		put(own + j, w);
-		if (two) put(own + j2, w2);
-	}
+	fetch<1>(a, bs * S.nHalo, words, tag, [&](int j) { return bs * halo[j / bs] + j % bs; },
+			 [&](int j, const ResWord(&w)[1]) { put(bs * S.L.nOwn + j, w[0]); });
 }
 
 // Row warps, the first `warps` of which have rows: leaves the warp's FP64 sums of NV (1 or 2) values a thread
@@ -496,48 +498,64 @@ __device__ __forceinline__ Talk open_talk(const ResArgs& a, const ResPart& p, in
 	return T;
 }
 
-// Sends the two words v0, v1 (the same in every lane) to every CTA of the system.
-__device__ __forceinline__ void send(const Talk& T, unsigned ph, unsigned tag, const unsigned (&v0)[3], const unsigned (&v1)[3])
+// Sends word {a, b, c} of the lanes 0-15 (0) and 16-31 (1; the same in every lane of a half) to every CTA of the system.
+__device__ __forceinline__ void send(const Talk& T, unsigned ph, unsigned tag, unsigned a, unsigned b, unsigned c)
 {
-	for (int j = threadIdx.x & 31; j < T.g; j += 32)
-	{
-		ResWord* box = T.out + ((ph & 1) ? T.parity : 0) + j * T.inStep;
-		st_word(&box[0], v0[0], v0[1], v0[2], tag);
-		st_word(&box[1], v1[0], v1[1], v1[2], tag);
-	}
+	const int lane = threadIdx.x & 31;
+	ResWord* box = T.out + ((ph & 1) ? T.parity : 0) + (lane & 15) * T.inStep + (lane >> 4);
+#pragma unroll 1
+	for (int j = lane & 15; j < T.g; j += 16, box += 16 * T.inStep) st_word(box, a, b, c, tag);
 }
 
 // Waits for every CTA's words of this phase, word 0 in lanes 0-15 and word 1 in lanes 16-31; use(word) is
-// called for the CTAs lane % 16, lane % 16 + 16, ... in order.
+// called for the CTAs lane % 16, lane % 16 + 16, ... in order. A poll loads the R words a lane needs of up to
+// 16 R CTAs and no more: with eight for every system a solve of 80 nodes took 0.469 ms, with four 0.415.
+template <int R, typename F>
+__device__ __forceinline__ bool receive_words(const ResArgs& a, const ResWord* box, int n, unsigned tag, F use)
+{
+	ResWord w[R];
+	Patience wait;
+	for (;;)
+	{
+#pragma unroll
+		for (int r = 0; r < R; ++r) w[r] = ld_word(box + (r < R - 1 || 16 * r < n ? 32 * r : 0));
+		bool all = true;
+#pragma unroll
+		for (int r = 0; r < R; ++r) all = all && w[r].tag == tag;
+		if (__all_sync(kFull, all || n <= 0)) break;
+		if (__any_sync(kFull, wait.lost(a)))
+		{
+			sh.bad = 1;
+			return false;
+		}
+	}
+#pragma unroll
+	for (int r = 0; r < R; ++r)
+		if (16 * r < n) use(w[r]);
+	return true;
+}
 template <typename F>
 __device__ __forceinline__ void receive(const ResArgs& a, const Talk& T, unsigned ph, unsigned tag, F use)
 {
-	constexpr int kRounds = 4;  // words in flight a lane: 64 CTAs at a time
-	const int lane = threadIdx.x & 31;
-	const ResWord* box = T.in + ((ph & 1) ? T.parity : 0) + 2 * (lane & 15) + (lane >> 4);
-	for (int j0 = lane & 15; j0 - (lane & 15) < T.g; j0 += 16 * kRounds, box += 32 * kRounds)
+	const int lane = threadIdx.x & 31, j = lane & 15;
+	const ResWord* box = T.in + ((ph & 1) ? T.parity : 0) + (lane >> 4);
+#pragma unroll 1
+	for (int first = 0; first < T.g; first += 64)
 	{
-		ResWord w[kRounds];
-		Patience wait;
-		for (;;)
-		{
-			bool all = true;
-#pragma unroll
-			for (int r = 0; r < kRounds; ++r)
-				if (j0 + 16 * r < T.g) w[r] = ld_word(box + 32 * r);
-#pragma unroll
-			for (int r = 0; r < kRounds; ++r)
-				if (j0 + 16 * r < T.g) all = all && w[r].tag == tag;
-			if (__all_sync(kFull, all)) break;
-			if (__any_sync(kFull, wait.lost(a)))
-			{
-				sh.bad = 1;
-				return;
-			}
-		}
-#pragma unroll
-		for (int r = 0; r < kRounds; ++r)
-			if (j0 + 16 * r < T.g) use(w[r]);
+		// Lanes past the last CTA read CTA 0's word (first, in a later batch) and leave it out.
+		const int n = T.g - first - j;
+		const ResWord* from = box + 2 * (n > 0 ? first + j : 0);
+		const int rounds = min(4, (T.g - first + 15) / 16);
+		bool ok;
+		if (rounds == 1)
+			ok = receive_words<1>(a, from, n, tag, use);
+		else if (rounds == 2)
+			ok = receive_words<2>(a, from, n, tag, use);
+		else if (rounds == 3)
+			ok = receive_words<3>(a, from, n, tag, use);
+		else
+			ok = receive_words<4>(a, from, n, tag, use);
+		if (!ok) return;
 	}
 }
 
@@ -554,16 +572,8 @@ __device__ __forceinline__ void total_f64(const ResArgs& a, const Talk& T, unsig
 		if (o < T.nSums) t += __shfl_xor_sync(kFull, t, o);
 	if (T.g > 1)
 	{
-		unsigned out[2][3];
-#pragma unroll
-		for (int k = 0; k < 2; ++k)
-		{
-			const unsigned long long u = (unsigned long long)__double_as_longlong(__shfl_sync(kFull, t, 16 * k));
-			out[k][0] = (unsigned)u;
-			out[k][1] = (unsigned)(u >> 32);
-			out[k][2] = 0u;
-		}
-		send(T, ph, tag, out[0], out[1]);
+		const unsigned long long u = (unsigned long long)__double_as_longlong(__shfl_sync(kFull, t, lane & 16));
+		send(T, ph, tag, (unsigned)u, (unsigned)(u >> 32), 0u);
 		during();
 		t = 0.0;
 		receive(a, T, ph, tag, [&](const ResWord& w) {
@@ -601,16 +611,9 @@ __device__ __forceinline__ void total_pairs(const ResArgs& a, const Talk& T, uns
 	if (T.g > 1)
 	{
 		// Words {r.u, |r|^2 high}, {w.u, |r|^2 low}.
-		unsigned out[2][3];
-#pragma unroll
-		for (int k = 0; k < 2; ++k)
-		{
-			out[k][0] = __float_as_uint(__shfl_sync(kFull, t.h, 16 * k));
-			out[k][1] = __float_as_uint(__shfl_sync(kFull, t.l, 16 * k));
-		}
-		out[0][2] = __float_as_uint(__shfl_sync(kFull, t2.h, 0));
-		out[1][2] = __float_as_uint(__shfl_sync(kFull, t2.l, 0));
-		send(T, ph, tag, out[0], out[1]);
+		const int from = lane & 16;  // the lanes that hold the sums whatever the number of warps
+		send(T, ph, tag, __float_as_uint(__shfl_sync(kFull, t.h, from)), __float_as_uint(__shfl_sync(kFull, t.l, from)),
+			 __float_as_uint(__shfl_sync(kFull, half ? t2.l : t2.h, from)));
 		during();
 		t = t2 = {0.f, 0.f};
 		receive(a, T, ph, tag, [&](const ResWord& w) {
@@ -703,6 +706,7 @@ __device__ __forceinline__ unsigned talk_mixed(const ResArgs& a, const ResPart p
 	for (int it = 0; mode != 3; ++it)
 	{
 		++ph;
+		bool lost = false;  // looked up while words travel; a wait that gives up after that ends the next phase
 		beat(a, p, ph);
 		sums_wait();
 		if (mode == 1)
@@ -737,6 +741,7 @@ __device__ __forceinline__ unsigned talk_mixed(const ResArgs& a, const ResPart p
 			Pair v[3], rzInv{}, back{};
 			const bool first = mode == 2 && updates == 0;
 			total_pairs(a, T, ph, base + ph, v, [&] {
+				lost = given_up();
 				rzInv = Pair{1.f, 0.f} / (mode == 2 ? rzPend * ratioP * ratioP : rz);
 				back = rzInv / alpha;
 			});
@@ -768,7 +773,7 @@ __device__ __forceinline__ unsigned talk_mixed(const ResArgs& a, const ResPart p
 				mode = nonfinite ? 3 : 0;
 			}
 		}
-		if (it + 1 >= maxLoop || given_up()) mode = 3;
+		if (it + 1 >= maxLoop || lost) mode = 3;
 		publish(mode);
 	}
 	if (p.rank == 0 && (threadIdx.x & 31) == 0) write_result(a, p, 0, bb[0], rrTrue, iter, updates, converged, nonfinite);
@@ -896,7 +901,7 @@ __device__ __forceinline__ void multiply(const MixedShare& S, const float4* U, i
 		// A plain loop: rounds of guarded loads took twice as long in shared memory (19 slots: 2,680 cycles of a
 		// warp, here 1,410; 15 warps at once are bound by the shared-memory pipe's 14 words a slot).
 		constexpr bool kFar = std::is_same<std::decay_t<decltype(slots)>, FarSlots>::value;
-		constexpr int kUnroll = kFar ? 2 : 6;  // far slots: 12.0 ms a solve of 270,641 nodes at 2, 12.7 at 3, 12.4 at 4
+		constexpr int kUnroll = kFar ? 3 : 6;  // far slots: 12.9 ms a solve of 270,641 nodes at 2, 12.6 at 3, 13.4 at 4
 #pragma unroll kUnroll
 		for (int k = 0; k < n; ++k)
 		{
@@ -1259,9 +1264,10 @@ __device__ __forceinline__ unsigned talk_f64(const ResArgs& a, const ResPart p, 
 		beat(a, p, ph);
 		sums_wait();
 		double pq[1], rzInv = 0.0;
-		total_f64<1>(a, T, ph, base + ph, pq, [] {});
+		bool lost = false;  // as in talk_mixed
+		total_f64<1>(a, T, ph, base + ph, pq, [&] { lost = given_up(); });
 		sh.alpha = rz / pq[0];
-		if (given_up())
+		if (lost)
 		{
 			converged = 0;
 			publish(3);
@@ -1270,7 +1276,10 @@ __device__ __forceinline__ unsigned talk_f64(const ResArgs& a, const ResPart p, 
 		publish(0);
 		++ph;
 		sums_wait();
-		total_f64<2>(a, T, ph, base + ph, v, [&] { rzInv = 1.0 / rz; });
+		total_f64<2>(a, T, ph, base + ph, v, [&] {
+			rzInv = 1.0 / rz;
+			lost = given_up();
+		});
 		rr = v[0];
 		// rr >= 0 and the threshold compare as integers (no FP64 instruction); NaN and infinity are above.
 		const long long bits = __double_as_longlong(rr) & 0x7fffffffffffffffLL;
@@ -1292,7 +1301,7 @@ __device__ __forceinline__ unsigned talk_f64(const ResArgs& a, const ResPart p, 
 				mode = 3;
 			}
 		}
-		if (given_up()) mode = 3;
+		if (lost) mode = 3;
 		publish(mode);
 	}
 	if (p.rank == 0 && (threadIdx.x & 31) == 0) write_result(a, p, rhs, bb, rr, iter, 0, converged, !isfinite(rr));
