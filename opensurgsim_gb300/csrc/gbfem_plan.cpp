@@ -159,7 +159,7 @@ std::vector<int> res_widths(int form, double local, const std::vector<long long>
 	// Where CTAs are left over, shares shrink to this weight: below it an iteration is all exchange (18,081
 	// nodes, mixed: 0.56 ms a solve at 60, 0.53 at 80, 0.56 at 100, 0.68 at 200; 1,331 nodes, FP64: 0.58 ms at 14,
 	// 0.65 at 20, 0.82 at 50; 17,280 scalar rows: 0.54 ms at 126, 0.50 at 250, 0.56 at 400, 0.62 at 600).
-	const double least = res_mixed(form) ? 50.0 : (form == kResF64S ? 200.0 : 14.0);
+	const double least = res_mixed(form) ? 45.0 : (form == kResF64S ? 200.0 : 14.0);
 	std::vector<int> width(nseg);
 	long long total = 0;
 	for (int s = 0; s < nseg; ++s)

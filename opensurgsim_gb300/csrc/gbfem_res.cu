@@ -787,7 +787,8 @@ __device__ __forceinline__ unsigned talk_mixed(const ResArgs& a, const ResPart p
 struct MixedShare
 {
 	ResLayout L;
-	int c0, nHalo, first, last;  // this warp's entries of the chunk list
+	int c0, nHalo, first, last;  // this warp's entries of the chunk list,
+	int head;                    // the chunk of the first
 	int colKept;                 // shared offset of the kept columns
 	unsigned long long policy;   // L2 policy of the slots read in every product
 	const float* val;            // the share's first slot
@@ -826,6 +827,7 @@ __device__ __forceinline__ MixedShare open_mixed(const ResArgs& a, const ResPart
 	for (int i = tid; i < S.nHalo; i += kRowThreads) halo[i] = a.halo[p.h0 + i];
 	S.first = a.chunkWarp[p.warp0 + w];
 	S.last = a.chunkWarp[p.warp0 + w + 1];
+	S.head = S.first < S.last ? a.chunkList[S.first] : 0;
 	for (int j = S.first; j < S.last; ++j)
 	{
 		const int c = a.chunkList[j], o = a.off[p.c0 + c] - k0, o1 = a.off[p.c0 + c + 1] - k0;
@@ -1187,10 +1189,12 @@ __device__ __forceinline__ void rows_mixed(const ResArgs& a, const ResPart p, un
 		// w of the own rows; r.u, w.u, |r|^2: FP32 over a chunk's rows, pairs over chunks, warps and CTAs.
 		ResWord* words = a.rowWords + ((ph & 1) ? (size_t)a.nrows : 0);
 		Pair sum[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+		int next = S.head;  // chunks are looked up one ahead
 #pragma unroll 1
 		for (int j = S.first; j < S.last; ++j)
 		{
-			const int c = a.chunkList[j], i = 32 * c + lane;
+			const int c = next, i = 32 * c + lane;
+			if (j + 1 < S.last) next = a.chunkList[j + 1];
 			float w0 = 0.f, w1 = 0.f, w2 = 0.f;
 			multiply(S, U, c, w0, w1, w2);
 			if (!alone) send_xyz(&words[row0 + i], w0, w1, w2, tag);
