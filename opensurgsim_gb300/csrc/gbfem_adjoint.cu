@@ -25,9 +25,9 @@ namespace {
 
 constexpr int kAdjThreads = 64;
 
-// One thread per element, its passes in turn (splitting them over threads was measured slower:
-// every pass needs the same large per-thread state). gx[e*12 + 0..11], gv[e*12 + 0..11]; gLogE[e],
-// gNu[e] accumulate.
+// One thread per element, its passes in turn, or (grid rows) a few of them: the dual passes spread over all rows but
+// the last, which has the moduli's. gx[e*12 + 3..11] (an element's node 0 has minus the sum of the others: the
+// gather forms it), gv[e*12 + 0..11]; gLogE[e], gNu[e] accumulate.
 template <typename S>
 __global__ void __launch_bounds__(kAdjThreads) k_element_adjoint(DevBody b, const double* __restrict__ x,
 																 const double* __restrict__ v,
@@ -39,6 +39,10 @@ __global__ void __launch_bounds__(kAdjThreads) k_element_adjoint(DevBody b, cons
 {
 	const int e = blockIdx.x * blockDim.x + threadIdx.x;
 	if (e >= b.E) return;
+	// Passes of this block: all, or those of its row of the grid (the last row: the moduli's).
+	const int rows = gridDim.y, first = rows == 1 ? 0 : blockIdx.y * 9 / (rows - 1),
+			  last = rows == 1 ? 9 : (blockIdx.y == rows - 1 ? 9 : (blockIdx.y + 1) * 9 / (rows - 1));
+	const bool tail = rows == 1 || blockIdx.y == rows - 1;
 	const int E = b.E;
 	const int4 t4 = b.tets[e];
 	const int nd[4] = {t4.x, t4.y, t4.z, t4.w};
@@ -64,8 +68,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_element_adjoint(DevBody b, cons
 	const bool moduli = gLogE || gNu;
 	double pl = 0.0, pm = 0.0;
 	adj::element_adjoint<S>(nd, X, R0, V, MU, DV, g, lamV, muV, cm, dt, alpha, beta, gx + (size_t)e * 12,
-							gv + (size_t)e * 12, moduli ? &pl : nullptr, &pm, b.lumped != 0);
-	if (!moduli) return;
+							gv + (size_t)e * 12, moduli ? &pl : nullptr, &pm, b.lumped != 0, first, last, tail);
+	if (!moduli || !tail) return;
 	// lambda V and mu V are both proportional to E: d/d log E scales each by one.
 	if (gLogE) gLogE[e] += lamV * pl + muV * pm;
 	if (gNu)
@@ -82,30 +86,23 @@ __global__ void k_adjoint_gather(DevBody b, const double* __restrict__ gx, const
 								 const double* __restrict__ lx, const double* __restrict__ lv, double dt,
 								 double* __restrict__ lxOut, double* __restrict__ lvOut)
 {
-	const int I = blockIdx.x * blockDim.x + threadIdx.x;
-	if (I >= b.N) return;
-	double sx[3] = {0, 0, 0}, sv[3] = {0, 0, 0};
+	const int d = blockIdx.x * blockDim.x + threadIdx.x;
+	if (d >= 3 * b.N) return;
+	const int I = d / 3, j = d - 3 * I;
+	double sx = 0.0, sv = 0.0;
 	const int k1 = b.iptr[I + 1];
+#pragma unroll 2
 	for (int k = b.iptr[I]; k < k1; ++k)
 	{
 		const int c = b.iidx[k];
 		const size_t o = (size_t)(c >> 2) * 12;
 		const int a = c & 3;
-#pragma unroll
-		for (int j = 0; j < 3; ++j)
-		{
-			sx[j] += (a == 0) ? -(gx[o + 3 + j] + gx[o + 6 + j] + gx[o + 9 + j]) : gx[o + 3 * a + j];
-			sv[j] += gv[o + 3 * a + j];
-		}
+		sx += (a == 0) ? -(gx[o + 3 + j] + gx[o + 6 + j] + gx[o + 9 + j]) : gx[o + 3 * a + j];
+		sv += gv[o + 3 * a + j];
 	}
-#pragma unroll
-	for (int j = 0; j < 3; ++j)
-	{
-		const int d = 3 * I + j;
-		const double l = lx[d];
-		lxOut[d] = l + sx[j];
-		lvOut[d] = dt * l + lv[d] + sv[j];
-	}
+	const double l = lx[d];
+	lxOut[d] = l + sx;
+	lvOut[d] = dt * l + lv[d] + sv;
 }
 
 // Right-hand side of the transposed solve, g = dt lx + lv, zero on BC dofs.
@@ -159,11 +156,19 @@ void launch_element_adjoint(const DevBody& b, const double* x, const double* v, 
 							cudaStream_t s, bool fp32)
 {
 	if (b.E == 0) return;
+	// Rows of the grid: the passes of an element are independent but for its rotation, which every row forms again.
+	// Few elements leave the chip idle while a thread runs through all passes, and their FP64 instructions
+	// take 64 cycles each; the FP32 passes of many elements are better off with one rotation. Two-step rollouts with
+	// 1, 4 and 10 rows: FP64 625 elements 7.3, 4.7 and 3.9 ms, 6,000 8.0, 5.7 and 6.0, 80,000 28.1, 25.9 and
+	// 28.7; FP32 625 2.26, 2.14 and 2.07, 6,000 2.44, 2.37 and 2.38, 80,000 4.04, 3.94 and 4.47, 134,400 4.97,
+	// 5.01 and 5.93.
+	const int rows = b.E <= 2000 ? 10 : (!fp32 || b.E <= 100000 ? 4 : 1);
+	const dim3 grid(blocks_of(b.E, kAdjThreads), rows);
 	if (fp32)
-		k_element_adjoint<float><<<blocks_of(b.E, kAdjThreads), kAdjThreads, 0, s>>>(b, x, v, mu, dv, dt, alpha, beta,
+		k_element_adjoint<float><<<grid, kAdjThreads, 0, s>>>(b, x, v, mu, dv, dt, alpha, beta,
 																					 gx, gv, gLogE, gNu);
 	else
-		k_element_adjoint<double><<<blocks_of(b.E, kAdjThreads), kAdjThreads, 0, s>>>(b, x, v, mu, dv, dt, alpha, beta,
+		k_element_adjoint<double><<<grid, kAdjThreads, 0, s>>>(b, x, v, mu, dv, dt, alpha, beta,
 																					  gx, gv, gLogE, gNu);
 }
 
@@ -171,7 +176,7 @@ void launch_adjoint_gather(const DevBody& b, const double* gx, const double* gv,
 						   double dt, double* lxOut, double* lvOut, cudaStream_t s)
 {
 	if (b.N == 0) return;
-	k_adjoint_gather<<<blocks_of(b.N, 128), 128, 0, s>>>(b, gx, gv, lx, lv, dt, lxOut, lvOut);
+	k_adjoint_gather<<<blocks_of(3 * b.N, 192), 192, 0, s>>>(b, gx, gv, lx, lv, dt, lxOut, lvOut);
 }
 
 void launch_adjoint_rhs(int n, const uint8_t* bc, const double* lx, const double* lv, double dt, double* g,

@@ -185,12 +185,15 @@ __host__ __device__ inline int element_rotation(const int (&nd)[4], const double
 // S is the arithmetic of the passes: double (FP64 form) or float (mixed form, FP32 element math
 // with the corotated strain formed as in its forward step). The rotation, the passes' inputs and the
 // psi coefficients are formed once; a dual pass only moves its seed.
+// first, last: the dual passes to run (0..8; gx[0..2] only when all of them run); moduli: whether to run the two
+// passes of gv, pLam and pMu.
 template <typename S = double>
 __host__ __device__ inline void element_adjoint(const int (&nd)[4], const double (&X)[4][3], const double (&R0)[4][3],
 												const double (&V)[4][3], const double (&MU)[12], const double (&DV)[12],
 												const double (&g)[4][3], double lamV, double muV, double cm, double dt,
 												double alpha, double beta, double* gx, double* gv, double* pLam,
-												double* pMu, bool lumped = false)
+												double* pMu, bool lumped = false, int first = 0, int last = 9,
+												bool moduli = true)
 {
 	using D = ad::DualT<S>;
 	const double c2 = dt + beta;
@@ -212,7 +215,7 @@ __host__ __device__ inline void element_adjoint(const int (&nd)[4], const double
 		fill_input(in, nd, X, R0, V, dt, alpha, beta, -1, -1, lumped);
 		double sx[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
-		for (int item = 0; item < 9; ++item)
+		for (int item = first; item < last; ++item)
 		{
 			const int node = 1 + item / 3, axis = item % 3;
 #pragma unroll
@@ -226,8 +229,10 @@ __host__ __device__ inline void element_adjoint(const int (&nd)[4], const double
 			gx[3 + item] = d;
 			sx[axis] += d;
 		}
-		for (int k = 0; k < 3; ++k) gx[k] = -sx[k];
+		if (last - first == 9)
+			for (int k = 0; k < 3; ++k) gx[k] = -sx[k];
 	}
+	if (moduli)
 	{
 		// psi_e's elastic part and K_e are linear in (lambda V, mu V) (K0, the rotated stiffness and the
 		// rotation terms all are; R and the singular-G decision do not depend on the moduli): two passes
