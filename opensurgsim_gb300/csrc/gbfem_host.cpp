@@ -373,7 +373,7 @@ struct gbfem_handle_s
 	// Compliance (gbfem_apply_compliance): the system matrix of the last step, and its dt.
 	bool systemReady = false;
 	double lastDt = 0.0;
-	DevBuf<double> d_mcgVec, d_mcgPart, d_Re, d_Wn, d_xprev;
+	DevBuf<double> d_mcgVec, d_mcgPart, d_Qe, d_Wn, d_xprev;
 	DevBuf<McgCtl> d_mcgCtl;
 	McgCtl* h_mcgCtl = nullptr;
 	DevBuf<int> d_counters;
@@ -466,7 +466,7 @@ struct gbfem_handle_s
 		d_colX.free();
 		d_colSeg.free();
 		d_colErr.free();
-		for (auto* b : {&d_mcgVec, &d_mcgPart, &d_Re, &d_Wn, &d_xprev}) b->free();
+		for (auto* b : {&d_mcgVec, &d_mcgPart, &d_Qe, &d_Wn, &d_xprev}) b->free();
 		d_mcgCtl.free();
 		if (h_mcgCtl) cudaFreeHost(h_mcgCtl);
 		h_mcgCtl = nullptr;
@@ -2386,16 +2386,16 @@ gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double*
 	const DevBody body = h->body();
 	if (warp)
 	{
-		if (!h->d_Re.p)
+		if (!h->d_Qe.p)
 		{
-			GB_CUDA(h, h->d_Re.alloc(9 * (size_t)h->E));
+			GB_CUDA(h, h->d_Qe.alloc(4 * (size_t)h->E));
 			GB_CUDA(h, h->d_Wn.alloc(9 * (size_t)N));
 			GB_CUDA(h, h->d_xprev.alloc(n));
 		}
 		// The rotations of the last element update: at the positions the last step started from.
 		launch_prev_positions(n, h->d_x.p, h->d_v.p, h->lastDt, h->d_xprev.p, s);
-		launch_element_rotation(body, h->d_xprev.p, h->d_Re.p, s);
-		launch_node_rotation(body, h->d_Re.p, h->d_Wn.p, s);
+		launch_element_rotation(body, h->d_xprev.p, h->d_Qe.p, s);
+		launch_node_rotation(body, h->d_Qe.p, h->d_Wn.p, s);
 	}
 	double *B = h->d_mcgVec.p, *X = B + n8, *R = X + n8, *Z = R + n8, *P = Z + n8, *Q = P + n8;
 	const MatSellT<double> A64{h->nrows, h->d_perm.p, h->d_off.p, h->d_sellcol.p, h->d_A.p};

@@ -146,11 +146,11 @@ void launch_mcg_spmm(const MatSellT<double>* A64, const MatSellT<float>* A32, co
 void launch_mcg_update(int n, const double* invd64, const float* invd32, const double* P, const double* Q, double* X,
 					   double* R, double* Z, McgCtl* ctl, double* part, const Launch& L);
 void launch_mcg_pupdate(int n, const double* Z, double* P, const McgCtl* ctl, const Launch& L);
-// Per-element rotation of the polar decomposition at positions x (9 per element, row-major).
-void launch_element_rotation(const DevBody& b, const double* x, double* Re, cudaStream_t s);
+// Per-element rotation of the polar decomposition at positions x, as a unit quaternion (4 per element).
+void launch_element_rotation(const DevBody& b, const double* x, double* Qe, cudaStream_t s);
 // Per-node warping rotation: the running slerp average of the node's element rotations in element
 // order (Fem3DCorotationalTetrahedronRepresentation.cpp:112-140).
-void launch_node_rotation(const DevBody& b, const double* Re, double* Wn, cudaStream_t s);
+void launch_node_rotation(const DevBody& b, const double* Qe, double* Wn, cudaStream_t s);
 // out = x - dt v (the positions a step started from, after x = x_t + dt v).
 void launch_prev_positions(int n, const double* x, const double* v, double dt, double* out, cudaStream_t s);
 // X (n x kMcgCols, interleaved) <- blockdiag(W) X, or its transpose.

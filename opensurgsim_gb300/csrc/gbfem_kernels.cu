@@ -884,31 +884,6 @@ __global__ void k_mcg_pupdate(int n, const double* __restrict__ Z, double* __res
 		}
 }
 
-// Rotation of every element at positions x (the polar factor of the corotational update).
-__global__ void k_element_rotation(DevBody b, const double* __restrict__ x, double* __restrict__ Re)
-{
-	const int e = blockIdx.x * blockDim.x + threadIdx.x;
-	if (e >= b.E) return;
-	const int E = b.E;
-	const int4 t4 = b.tets[e];
-	const int nd[4] = {t4.x, t4.y, t4.z, t4.w};
-	double F[9];
-#pragma unroll
-	for (int i = 0; i < 3; ++i)
-#pragma unroll
-		for (int j = 0; j < 3; ++j)
-		{
-			double s = 0.0;
-#pragma unroll
-			for (int a = 1; a < 4; ++a) s += (x[3 * nd[a] + i] - x[3 * nd[0] + i]) * b.rest[(3 * a + j) * E + e];
-			F[3 * i + j] = s;
-		}
-	double R[9];
-	if (!elem::polar_newton(F, R)) elem::polar_svd(F, R);
-#pragma unroll
-	for (int k = 0; k < 9; ++k) Re[(size_t)e * 9 + k] = R[k];
-}
-
 // Unit quaternion (w, x, y, z) of a rotation matrix (row-major), by the largest of the four
 // diagonal combinations (numerically stable for every rotation).
 __device__ void quat_from_matrix(const double* R, double* q)
@@ -948,6 +923,30 @@ __device__ void quat_from_matrix(const double* R, double* q)
 	}
 }
 
+// Rotation of every element at positions x (the polar factor of the corotational update) as a unit quaternion.
+__global__ void k_element_rotation(DevBody b, const double* __restrict__ x, double* __restrict__ Qe)
+{
+	const int e = blockIdx.x * blockDim.x + threadIdx.x;
+	if (e >= b.E) return;
+	const int E = b.E;
+	const int4 t4 = b.tets[e];
+	const int nd[4] = {t4.x, t4.y, t4.z, t4.w};
+	double F[9];
+#pragma unroll
+	for (int i = 0; i < 3; ++i)
+#pragma unroll
+		for (int j = 0; j < 3; ++j)
+		{
+			double s = 0.0;
+#pragma unroll
+			for (int a = 1; a < 4; ++a) s += (x[3 * nd[a] + i] - x[3 * nd[0] + i]) * b.rest[(3 * a + j) * E + e];
+			F[3 * i + j] = s;
+		}
+	double R[9];
+	elem::rotation_fp64(F, R);
+	quat_from_matrix(R, Qe + (size_t)e * 4);
+}
+
 __device__ void matrix_from_quat(const double* q, double* R)
 {
 	const double w = q[0], x = q[1], y = q[2], z = q[3];
@@ -962,50 +961,70 @@ __device__ void matrix_from_quat(const double* q, double* R)
 	R[8] = 1 - 2 * (x * x + y * y);
 }
 
-// Spherical linear interpolation from a to b at t along the shorter arc (linear weights when the
-// quaternions are within one rounding unit of each other).
-__device__ void quat_slerp(const double* a, const double* b, double t, double* out)
+// sin(u th) / sin(th) for the angle th with cos(th) = c >= 0: the weight of an end of a spherical interpolation. Near
+// c = 1, where neighbouring elements' rotations are, by the series in c - 1 (D. Eberly, "A Fast and Accurate
+// Algorithm for Computing SLERP", 2011: a_0 = u, a_i = a_(i-1) (u^2 - i^2) / (i (2 i + 1))), whose terms fall by more
+// than 200 each for 1 - c <= 0.01: eight leave 1e-18. It has no inverse cosine, sine or division.
+__device__ __forceinline__ double slerp_weight(double u, double c)
 {
-	const double d = a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3];
-	const double ad = fabs(d);
-	double s0, s1;
-	if (ad >= 1.0 - DBL_EPSILON)
+	const double x = c - 1.0;
+	if (x >= -0.01)
 	{
-		s0 = 1.0 - t;
-		s1 = t;
-	}
-	else
-	{
-		const double th = acos(ad), st = sin(th);
-		s0 = sin((1.0 - t) * th) / st;
-		s1 = sin(t * th) / st;
-	}
-	if (d < 0.0) s1 = -s1;
+		const double u2 = u * u;
+		double s = 1.0;
 #pragma unroll
-	for (int k = 0; k < 4; ++k) out[k] = s0 * a[k] + s1 * b[k];
+		for (int i = 8; i >= 1; --i) s = fma((u2 - double(i * i)) * (1.0 / double(i * (2 * i + 1))) * x, s, 1.0);
+		return u * s;
+	}
+	const double th = acos(c);
+	return sin(u * th) / sin(th);
 }
 
-__global__ void k_node_rotation(DevBody b, const double* __restrict__ Re, double* __restrict__ Wn)
+// 1 / i for the position of an element at its node (an FP64 division takes 565 cycles).
+struct Inverses
 {
-	const int I = blockIdx.x * blockDim.x + threadIdx.x;
-	if (I >= b.N) return;
-	const int k0 = b.iptr[I], k1 = b.iptr[I + 1];
-	double R[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-	if (k1 > k0)
+	double v[64];
+	constexpr Inverses() : v()
 	{
-		double q[4];
-		quat_from_matrix(Re + (size_t)(b.iidx[k0] >> 2) * 9, q);
-		for (int k = k0 + 1; k < k1; ++k)
-		{
-			double qe[4], qn[4];
-			quat_from_matrix(Re + (size_t)(b.iidx[k] >> 2) * 9, qe);
-			const double i = double(k - k0 + 1);  // the element's 1-based position at this node
-			quat_slerp(q, qe, 1.0 - 1.0 / i, qn);
-#pragma unroll
-			for (int m = 0; m < 4; ++m) q[m] = qn[m];
-		}
-		matrix_from_quat(q, R);
+		for (int i = 1; i < 64; ++i) v[i] = 1.0 / i;
 	}
+};
+__constant__ Inverses kInverse = Inverses();
+
+// Rotation of every node: the running spherical average of its elements' rotations in element order, along the
+// shorter arcs. Two threads a node, each with half of the quaternion and one of the two weights; the chain over the
+// ~20 elements of a node is FP64 instructions at 64 cycles each (205 us for 1,331 nodes with a thread a node, the
+// quaternions formed in the chain and the weights by acos and sin; 57 us here).
+__global__ void k_node_rotation(DevBody b, const double* __restrict__ Qe, double* __restrict__ Wn)
+{
+	const int t = blockIdx.x * blockDim.x + threadIdx.x, I = min(t >> 1, b.N - 1), half = t & 1;
+	const int k0 = b.iptr[I], k1 = b.iptr[I + 1];
+	const unsigned pair = 3u << (threadIdx.x & 30);  // this node's two lanes
+	const double2* Q = reinterpret_cast<const double2*>(Qe);
+	double2 q = half == 0 ? make_double2(1.0, 0.0) : make_double2(0.0, 0.0);
+	if (k1 > k0) q = Q[2 * (size_t)(b.iidx[k0] >> 2) + half];
+	double2 next = k0 + 1 < k1 ? Q[2 * (size_t)(b.iidx[k0 + 1] >> 2) + half] : q;
+	for (int k = k0 + 1; k < k1; ++k)
+	{
+		const double2 e = next;
+		if (k + 1 < k1) next = Q[2 * (size_t)(b.iidx[k + 1] >> 2) + half];
+		const int i = k - k0 + 1;  // the element's 1-based position at this node
+		const double inv = i < 64 ? kInverse.v[i] : 1.0 / double(i);
+		double d = q.x * e.x + q.y * e.y;
+		d += __shfl_xor_sync(pair, d, 1);
+		// The average so far has weight 1 / i of the arc, the element the rest.
+		double w = slerp_weight(half == 0 ? inv : 1.0 - inv, fabs(d));
+		if (half == 1 && d < 0.0) w = -w;
+		const double other = __shfl_xor_sync(pair, w, 1);
+		const double w0 = half == 0 ? w : other, w1 = half == 0 ? other : w;
+		q.x = w0 * q.x + w1 * e.x;
+		q.y = w0 * q.y + w1 * e.y;
+	}
+	const double2 o = make_double2(__shfl_xor_sync(pair, q.x, 1), __shfl_xor_sync(pair, q.y, 1));
+	if (half == 1 || (t >> 1) >= b.N) return;
+	const double all[4] = {q.x, q.y, o.x, o.y};
+	double R[9];
+	matrix_from_quat(all, R);
 #pragma unroll
 	for (int m = 0; m < 9; ++m) Wn[(size_t)I * 9 + m] = R[m];
 }
@@ -1232,16 +1251,16 @@ void launch_mcg_pupdate(int n, const double* Z, double* P, const McgCtl* ctl, co
 	k_mcg_pupdate<<<L.vecGrid, kVecThreads, 0, L.stream>>>(n, Z, P, ctl);
 }
 
-void launch_element_rotation(const DevBody& b, const double* x, double* Re, cudaStream_t s)
+void launch_element_rotation(const DevBody& b, const double* x, double* Qe, cudaStream_t s)
 {
 	if (b.E == 0) return;
-	k_element_rotation<<<blocks(b.E, 128), 128, 0, s>>>(b, x, Re);
+	k_element_rotation<<<blocks(b.E, 128), 128, 0, s>>>(b, x, Qe);
 }
 
-void launch_node_rotation(const DevBody& b, const double* Re, double* Wn, cudaStream_t s)
+void launch_node_rotation(const DevBody& b, const double* Qe, double* Wn, cudaStream_t s)
 {
 	if (b.N == 0) return;
-	k_node_rotation<<<blocks(b.N, 128), 128, 0, s>>>(b, Re, Wn);
+	k_node_rotation<<<blocks(2LL * b.N, 64), 64, 0, s>>>(b, Qe, Wn);
 }
 
 void launch_apply_node_rotation(int N, const double* Wn, double* X, bool transpose, cudaStream_t s)
