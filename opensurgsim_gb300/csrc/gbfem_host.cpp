@@ -72,7 +72,7 @@ cudaError_t res_budget(int device, int* smCount, int* budget)
 	int smem = 0;
 	cudaError_t e = cudaDeviceGetAttribute(smCount, cudaDevAttrMultiProcessorCount, device);
 	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
-	*budget = (smem - 2048) / 128 * 128;
+	*budget = (smem - 3072) / 128 * 128;
 	return e;
 }
 
@@ -81,6 +81,7 @@ struct ResDevice
 {
 	ResPlan plan;  // without its halo and column lists, which only the device reads
 	int maxRhs = 0;
+	bool cluster = false;  // one system of few CTAs: launched as one cluster
 	size_t smem = 0;
 	DevBuf<ResPart> parts;
 	DevBuf<int> halo, warp, list;
@@ -104,6 +105,8 @@ struct ResDevice
 		if (e == cudaSuccess) e = lcol.upload(plan.lcol.data(), plan.lcol.size(), s);
 		smem = res_smem(plan, plan.form, off, budget);
 		if (e == cudaSuccess) e = raise_res_smem_limit(smem, plan.form);
+		cluster = e == cudaSuccess && rhs == 1 && plan.segPart.size() == 2 &&
+				  res_cluster_fits(plan.form, (int)plan.parts.size(), smem);
 		if (e == cudaSuccess) e = cudaStreamSynchronize(s);
 		for (auto* v : {&plan.halo, &plan.chunkWarp, &plan.chunkList}) std::vector<int>().swap(*v);
 		std::vector<uint16_t>().swap(plan.lcol);
@@ -119,6 +122,7 @@ struct ResDevice
 		a.chunkList = list.p;
 		a.lcol = lcol.p;
 		a.smemBudget = (int)smem;
+		a.cluster = cluster;
 	}
 	cudaError_t launch(const ResArgs& a, int ctas, cudaStream_t s) const
 	{

@@ -156,9 +156,11 @@ std::vector<int> res_widths(int form, double local, const std::vector<long long>
 	const int vecs = (int)(local * res_loc_bytes(form)) + res_own_bytes(form) + 4;
 	const int slot = res_layout(form, 1, 0).slotBytes;
 	const double room = smemBudget - (kResPieces * 32.0 * res_part_bytes(form) + 2048.0);
-	// Where CTAs are left over, shares shrink to this weight: below it an iteration is all exchange (18,081
-	// nodes, mixed: 0.56 ms a solve at 60, 0.53 at 80, 0.56 at 100, 0.68 at 200; 1,331 nodes, FP64: 0.58 ms at 14,
-	// 0.65 at 20, 0.82 at 50; 17,280 scalar rows: 0.54 ms at 126, 0.50 at 250, 0.56 at 400, 0.62 at 600).
+	// Where CTAs are left over, shares shrink to this weight: below it an iteration is all exchange (mixed, 1,331
+	// nodes: 0.254 ms a solve at 40, 0.265 at 50, 0.279 at 80, 0.304 at 120; 216 nodes 0.230 at 40, 0.217 at 50;
+	// FP64 1,331 nodes: 0.58 ms at 14, 0.65 at 20, 0.82 at 50; 17,280 scalar rows: 0.54 ms at 126, 0.50 at 250,
+	// 0.56 at 400). Past 128 CTAs the sums take a third poll (18,081 nodes: 0.415 ms on 128, 0.443 on 152; FP64
+	// 29,184 nodes 1.19 and 1.23).
 	const double least = res_mixed(form) ? 45.0 : (form == kResF64S ? 200.0 : 14.0);
 	std::vector<int> width(nseg);
 	long long total = 0;
@@ -172,7 +174,13 @@ std::vector<int> res_widths(int form, double local, const std::vector<long long>
 	for (int s = 0; s < nseg; ++s)
 	{
 		const int most = std::max(1, std::min({ctas, 128, segChunks[s], (int)(segWeight[s] / least)}));
+		const int need = width[s];
 		if (spare > 1.0) width[s] = std::max(width[s], std::min(most, (int)(width[s] * spare)));
+		// One cluster rather than a few CTAs more: its exchanges are shorter (mixed 1,728 nodes 0.232 ms a solve on
+		// 16 CTAs, 0.258 on 20; 2,744 0.266 and 0.270 on 32; 3,024 0.281 and 0.274 on 35; FP64 576 nodes 0.404 on 16
+		// and 0.473 on 18, 729 0.497 and 0.473 on 23).
+		if (nseg == 1 && need <= kResCluster && width[s] > kResCluster && width[s] <= (res_mixed(form) ? 32 : 20))
+			width[s] = kResCluster;
 		width[s] = std::min(width[s], kResMaxGroup);
 	}
 	return width;

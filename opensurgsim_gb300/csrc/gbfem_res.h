@@ -11,6 +11,7 @@ namespace gbfem {
 
 constexpr int kResRowWarps = 15;  // warps of a CTA that own rows; one more sums and talks to the other CTAs
 constexpr int kResThreads = 32 * (kResRowWarps + 1);
+constexpr int kResCluster = 16;    // CTAs of a system that may run as one cluster
 constexpr int kResMaxGroup = 160;  // CTAs one system may spread over
 
 // One CTA's share of a system: a contiguous range of SELL-32 chunks, the rows of other CTAs its blocks
@@ -53,6 +54,7 @@ struct ResArgs
 	const int* perm;      // row position -> node (or scalar row), -1 on padding rows
 	const int* segMaxIter;  // per system, or null: maxIter
 	int maxIter, smemBudget;
+	int cluster;          // whether the launch is one system's CTAs as one cluster
 	float nearFraction;   // mixed forms: part of the slots beyond shared memory that L2 is to keep
 	double tol, drop;
 	long long timeoutNs;
@@ -134,6 +136,8 @@ __host__ __device__ inline ResLayout res_layout(int form, int nCh, int nHalo)
 }
 
 cudaError_t res_set_max_dynamic_smem(int form, int bytes);
+// Whether `ctas` CTAs with this much dynamic shared memory can run as one cluster.
+bool res_cluster_fits(int form, int ctas, size_t smem);
 cudaError_t res_launch(int form, int grid, size_t smem, const ResArgs& a, cudaStream_t s);
 
 }  // namespace gbfem
