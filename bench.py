@@ -161,12 +161,12 @@ def load_peak():
         return FALLBACK_HBM_GBS, "fallback"
 
 
-# FP64 arithmetic of the corotational element kernel (k_element_fp64), per tet: 1,717 DFMA, 742 DMUL
-# and 189 DADD executed (ncu counters sm__sass_thread_inst_executed_op_{dfma,dmul,dadd}_pred_on.sum
-# over one launch on the 10x10x10 cube, 5,000 tets) = 2 * 1717 + 742 + 189 FLOPs. The kernel does
+# FP64 arithmetic of the corotational element kernel (k_element_corot64), per tet: 826 DFMA, 401 DMUL
+# and 190 DADD executed (ncu counters sm__sass_thread_inst_executed_op_{dfma,dmul,dadd}_pred_on.sum
+# over one launch on the 10x10x10 cube, 5,000 tets) = 2 * 826 + 401 + 190 FLOPs. The kernel does
 # the polar decomposition, the corotational tangent and the force in closed form, so this is below
 # the reference's ~6-7k FMAs per tet for the same element update.
-ELEMENT_FP64_FLOPS_PER_TET = 2 * 1717 + 742 + 189
+ELEMENT_FP64_FLOPS_PER_TET = 2 * 826 + 401 + 190
 # GB300 FP64 (non-tensor) peak, NVIDIA's nominal figure; no measured FP64 peak is available.
 FP64_PEAK_TFLOPS = 1.25
 
@@ -222,6 +222,15 @@ def pin_schedule(body, args):
 
 def vector_passes(schedule):
     return 11 if schedule == 2 else 10
+
+
+def solve_roofline(schedule, traffic):
+    """Kernel, bound and DRAM traffic of the mixed solve. The one-phase schedule runs resident: its bytes are the
+    operands of its products, most of which shared memory and L2 serve, so their rate may pass HBM's."""
+    if schedule == 2:
+        return {"kernel": "k_res (resident mixed solve, one launch per step)",
+                "bound": "on chip (operand bytes against the measured HBM rate)", "traffic": None}
+    return {"kernel": "k_pcg_persistent (persistent mixed solve, one launch per step)", "bound": "hbm", "traffic": traffic}
 
 
 def bytes_per_iteration(nnz, N, s, vectors=10):
@@ -469,10 +478,9 @@ def run_batch(args, rank, world, local, dist):
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 2 * body.n * 8,
                 "d2h_bytes_per_step": 2 * body.n * 8},
         "roofline": {
-            "kernel": "k_pcg_persistent (whole batched mixed-precision solve, one launch per step)",
-            "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            **solve_roofline(tuning[3], load_traffic(f"pcg_persistent_batch{len(all_scenes)}") if world == 1 else None),
+            "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": (achieved / peak) if achieved else None,
-            "traffic": load_traffic(f"pcg_persistent_batch{len(all_scenes)}") if world == 1 else None,
             "algorithmic_bytes_per_launch": per_launch, "avg_launch_ms": launch_ms,
             "peak_source": f"{peak_kind} (hbm_gbs)",
             "bytes_model": (f"per mesh: CG iterations x (nnz*4 + nnz/9*4 + 4(N+1) + {vpass}*4*3N) + refreshes x "
@@ -534,7 +542,9 @@ def run_single(args, rank, world, local, dist):
     # The mixed form's steps run as a captured CUDA graph (the prescribed velocities are written into
     # the state between graph launches); the first warm-up step autotunes.
     graph = _lib.STEP_GRAPH if prec == _lib.PRECISION_MIXED else 0
-    flags = _lib.STEP_TIME_KERNELS | graph
+    # (Timing every product of an FP64 solve would take a single body off its resident solve: one step after
+    # the timed region does that.)
+    flags = graph if prec == _lib.PRECISION_FP64 else _lib.STEP_TIME_KERNELS | graph
     step = 0
     for w in range(args.warmup):
         set_driven(step)
@@ -589,6 +599,12 @@ def run_single(args, rank, world, local, dist):
     torch.cuda.synchronize(local)
     e2e_s = dist.reduce(time.perf_counter() - t0, "max")
     e2e_value = total_units / e2e_s
+    if prec == _lib.PRECISION_FP64:
+        set_driven(step)
+        body.step(dt, 1, _lib.STEP_TIME_KERNELS)
+        step += 1
+        for k in ("ms_spmv", "spmv_timed"):
+            agg[k] = body.stats()[k]
     fp64_alu = None
     if prec == _lib.PRECISION_FP64 and args.config != "hex":
         # The element kernel is bound by the FP64 pipe, not HBM: one more (untimed) step with phase
@@ -599,7 +615,7 @@ def run_single(args, rank, world, local, dist):
         el_ms = body.stats()["ms_element"]
         if el_ms > 0:
             tflops = m.num_tets * ELEMENT_FP64_FLOPS_PER_TET / (el_ms / 1e3) / 1e12
-            fp64_alu = {"kernel": "k_element_fp64", "bound": "fp64 pipe", "achieved": tflops,
+            fp64_alu = {"kernel": "k_element_corot64", "bound": "fp64 pipe", "achieved": tflops,
                         "peak": FP64_PEAK_TFLOPS, "unit": "TFLOP/s", "frac": tflops / FP64_PEAK_TFLOPS,
                         "flops_per_tet": ELEMENT_FP64_FLOPS_PER_TET, "launch_ms": el_ms,
                         "peak_source": "nominal (no measured FP64 peak)"}
@@ -619,7 +635,8 @@ def run_single(args, rank, world, local, dist):
         # Dominant kernel: the CG SpMV on the SELL-32 block matrix, timed per launch.
         spmv_bytes = body.nnz * 8 + (body.nnz // 9) * 4 + (body.num_nodes + 1) * 4 + 2 * body.n * 8
         launch_ms = agg["ms_spmv"] / max(1, agg["spmv_timed"])
-        kernel, per_launch, key = "k_cg_spmv_sell (fp64)", spmv_bytes, f"spmv_sell_fp64_{args.config}"
+        per_launch = spmv_bytes
+        roof = {"kernel": "k_cg_spmv_sell (fp64)", "bound": "hbm", "traffic": load_traffic(f"spmv_sell_fp64_{args.config}")}
         model = "nnz*8 + nnz/9*4 + 4(N+1) + 2*8*n per SpMV"
     else:
         # Dominant kernel: the persistent mixed-precision solve, one launch per step.
@@ -629,7 +646,7 @@ def run_single(args, rank, world, local, dist):
         vpass = vector_passes(body.tuning()[3])
         per_launch = (iters * bytes_per_iteration(body.nnz, body.num_nodes, 4, vpass)
                       + sweeps * bytes_per_refresh(body.nnz, body.num_nodes, 4) + 16 * body.n)
-        kernel, key = "k_pcg_persistent (mixed)", f"pcg_persistent_{args.config}"
+        roof = solve_roofline(body.tuning()[3], load_traffic(f"pcg_persistent_{args.config}"))
         model = (f"CG iterations x (nnz*4 + nnz/9*4 + 4(N+1) + {vpass}*4*n) + refreshes x (nnz*4 + nnz/9*4 + 4(N+1) "
                  "+ 3*8*n) + 16n")
     achieved = per_launch / (launch_ms / 1e3) / 1e9 if launch_ms > 0 else None
@@ -660,8 +677,8 @@ def run_single(args, rank, world, local, dist):
         "clocks": clocks,
         "e2e": {"value": e2e_value, "unit": unit, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "roofline": {
-            "kernel": kernel, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": (achieved / peak) if achieved else None, "traffic": load_traffic(key),
+            **roof, "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "frac": (achieved / peak) if achieved else None,
             "algorithmic_bytes_per_launch": per_launch, "avg_launch_ms": launch_ms,
             "peak_source": f"{peak_kind} (hbm_gbs)", "bytes_model": model,
         },
@@ -810,9 +827,10 @@ def run_bar_full(args, rank, world, local, dist):
                 "d2h_bytes_per_step": 2 * bm.n * 8,
                 "how": f"{e2e_steps} hold steps after the timed run, host clock"},
         "roofline": {
-            "kernel": "k_pcg_persistent (mixed)", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            **solve_roofline(tuning[3], load_traffic("pcg_persistent_bar")
+                             if abs(scene.mesh.h - BAR_H_WINDOW) < 1e-12 else None),
+            "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": (achieved / peak) if achieved else None,
-            "traffic": load_traffic("pcg_persistent_bar") if abs(scene.mesh.h - BAR_H_WINDOW) < 1e-12 else None,
             "algorithmic_bytes_per_launch": per_launch, "avg_launch_ms": solve_ms,
             "peak_source": f"{peak_kind} (hbm_gbs)",
             "bytes_model": (f"CG iterations x (nnz*4 + nnz/9*4 + 4(N+1) + {vpass}*4*n) + refreshes x "
