@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -2191,7 +2192,15 @@ gbfem_status create_impl(const gbfem_mesh_desc* meshes, int32_t count, const gbf
 		delete h;
 		return fail(nullptr, GBFEM_CUDA_ERROR, msg);
 	}
-	gbfem_status st = build_body(h, &merged);
+	gbfem_status st;
+	try
+	{
+		st = build_body(h, &merged);
+	}
+	catch (const std::bad_alloc&)
+	{
+		st = fail(h, GBFEM_OUT_OF_MEMORY, "out of host memory");
+	}
 	if (st != GBFEM_OK)
 	{
 		g_lastCreateError = h->err;
@@ -3527,7 +3536,14 @@ gbfem_status gbfem_cg_create(int32_t n, const int32_t* colptr, const int32_t* ro
 	if (e == cudaSuccess) e = g->invdiag.upload(invd.data(), n, g->stream);
 	for (auto* d : {&g->b, &g->x})
 		if (e == cudaSuccess) e = d->alloc(n);
-	if (e == cudaSuccess) e = cg_resident(g, cnt, colv, valv);
+	try
+	{
+		if (e == cudaSuccess) e = cg_resident(g, cnt, colv, valv);
+	}
+	catch (const std::bad_alloc&)
+	{
+		e = cudaErrorMemoryAllocation;
+	}
 	if (e == cudaSuccess && g->res.plan.ok)
 	{
 		*out = g;

@@ -5,9 +5,19 @@
 #include <algorithm>
 #include <cmath>
 #include <numeric>
+#include <utility>
 
 namespace gbfem {
 namespace {
+
+// Sorts indices by every third value from `coordinate`, then by index; the keys sit beside them for the sort.
+void sort_along(const double* coordinate, int* first, int* last)
+{
+	std::vector<std::pair<double, int>> key(last - first);
+	for (int* i = first; i != last; ++i) key[i - first] = {coordinate[3 * (size_t)*i], *i};
+	std::sort(key.begin(), key.end());
+	for (int* i = first; i != last; ++i) *i = key[i - first].second;
+}
 
 void bisect(const std::vector<double>& c, const std::vector<int>& w, int* first, int* last)
 {
@@ -24,10 +34,7 @@ void bisect(const std::vector<double>& c, const std::vector<int>& w, int* first,
 	int axis = 0;
 	for (int k = 1; k < 3; ++k)
 		if (hi[k] - lo[k] > hi[axis] - lo[axis]) axis = k;
-	std::sort(first, last, [&](int a, int b) {
-		const double u = c[3 * (size_t)a + axis], v = c[3 * (size_t)b + axis];
-		return u < v || (u == v && a < b);
-	});
+	sort_along(c.data() + axis, first, last);
 	long long total = 0, run = 0;
 	for (int i = 0; i < n; ++i) total += w[first[i]];
 	int cut = 0;
@@ -57,10 +64,7 @@ void split_nodes(const double* X, const std::vector<int>& w, int* first, int* la
 	int axis = 0;
 	for (int k = 1; k < 3; ++k)
 		if (hi[k] - lo[k] > hi[axis] - lo[axis]) axis = k;
-	std::sort(first, last, [&](int a, int b) {
-		const double u = X[3 * (size_t)a + axis], v = X[3 * (size_t)b + axis];
-		return u < v || (u == v && a < b);
-	});
+	sort_along(X + axis, first, last);
 	long long total = 0, run = 0;
 	for (int i = 0; i < n; ++i) total += w[first[i]];
 	const int gl = g / 2;
