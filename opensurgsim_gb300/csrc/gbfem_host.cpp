@@ -639,7 +639,7 @@ gbfem_status order_rows(gbfem_handle h, const double* X, bool compact, bool resi
 		segChunks[sg] = (h->segNode[sg + 1] - h->segNode[sg] + 31) / 32;
 		segWeight[sg] = (h->adjPtr[h->segNode[sg + 1]] - h->adjPtr[h->segNode[sg]]) / 32 + 1 + 4LL * segChunks[sg];
 	}
-	const std::vector<int> width = res_widths(form, compact ? 1.7 : 4.0, segWeight, segChunks, h->smCount, h->resBudget);
+	const std::vector<int> width = res_widths(form, compact ? 1.7 : 4.0, segWeight, segChunks, cost, h->smCount, h->resBudget);
 	std::vector<std::vector<int>> cut(nseg);
 	o.perm.clear();
 	o.segChunk.assign(nseg + 1, 0);
@@ -3412,7 +3412,7 @@ cudaError_t cg_resident(gbfem_cg g, const std::vector<int>& rowptr, const std::v
 		off[c + 1] = (int)slots;
 	}
 	if (slots * 32 > 2LL * rowptr[n] + 4096) return cudaSuccess;
-	const std::vector<int> width = res_widths(kResF64S, 4.0, {slots + 4LL * nch}, {nch}, g->smCount, budget);
+	const std::vector<int> width = res_widths(kResF64S, 4.0, {slots + 4LL * nch}, {nch}, {1.0}, g->smCount, budget);
 	std::vector<int> rcol(32 * slots), perm(32 * nch);
 	for (int c = 0; c < nch; ++c)
 		for (int l = 0; l < 32; ++l)

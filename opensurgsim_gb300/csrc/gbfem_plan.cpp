@@ -149,7 +149,7 @@ std::vector<int> res_chunk_order(const std::vector<double>& centroid, const std:
 }
 
 std::vector<int> res_widths(int form, double local, const std::vector<long long>& segWeight,
-							const std::vector<int>& segChunks, int ctas, int smemBudget)
+							const std::vector<int>& segChunks, const std::vector<double>& cost, int ctas, int smemBudget)
 {
 	const int nseg = (int)segWeight.size();
 	// Bytes of a row's vectors, its own and its part of the halo, and of a slot. A share takes up to `scale`
@@ -166,7 +166,7 @@ std::vector<int> res_widths(int form, double local, const std::vector<long long>
 	// 0.56 at 400). Past 128 CTAs the sums take a third poll (18,081 nodes: 0.415 ms on 128, 0.443 on 152; FP64
 	// 29,184 nodes 1.19 and 1.23).
 	const double least = res_mixed(form) ? 45.0 : (form == kResF64S ? 200.0 : 14.0);
-	std::vector<int> width(nseg);
+	std::vector<int> width(nseg), most(nseg);
 	long long total = 0;
 	for (int s = 0; s < nseg; ++s)
 	{
@@ -174,19 +174,42 @@ std::vector<int> res_widths(int form, double local, const std::vector<long long>
 		const double need = std::max(rows * vecs / 0.95, (rows * vecs + matrix) / scale) / room;
 		total += width[s] = std::max(1, std::min((int)(need * 1.02 + 1.0), std::min(ctas, segChunks[s])));
 	}
-	const double spare = (double)ctas / total;
 	for (int s = 0; s < nseg; ++s)
+		most[s] = std::max(width[s], std::min({ctas, 128, segChunks[s], (int)(segWeight[s] / least)}));
+	if (nseg == 1)
 	{
-		const int most = std::max(1, std::min({ctas, 128, segChunks[s], (int)(segWeight[s] / least)}));
-		const int need = width[s];
-		if (spare > 1.0) width[s] = std::max(width[s], std::min(most, (int)(width[s] * spare)));
 		// One cluster rather than a few CTAs more: its exchanges are shorter (mixed 1,728 nodes 0.232 ms a solve on
 		// 16 CTAs, 0.258 on 20; 2,744 0.266 and 0.270 on 32; 3,024 0.281 and 0.274 on 35; FP64 576 nodes 0.404 on 16
 		// and 0.473 on 18, 729 0.497 and 0.473 on 23).
-		if (nseg == 1 && need <= kResCluster && width[s] > kResCluster && width[s] <= (res_mixed(form) ? 32 : 20))
-			width[s] = kResCluster;
-		width[s] = std::min(width[s], kResMaxGroup);
+		const int need = width[0];
+		width[0] = most[0];
+		if (need <= kResCluster && width[0] > kResCluster && width[0] <= (res_mixed(form) ? 32 : 20)) width[0] = kResCluster;
 	}
+	else
+	{
+		// The CTAs left over go one by one to the system expected to end last: its iterations times an
+		// iteration's waits and its share's work (all systems widened alike: 36 FP64 meshes of 300 to 2,100 cubes
+		// 2.55 ms a solve, here 2.02; 16 of 800 to 4,000 2.54 and 2.14; 20 mixed ones of 500 to 12,500 1.21 and
+		// 0.92). Systems that take more CTAs than there are go in turn, the longest first: squeezing them into one
+		// turn was slower (24 FP64 meshes of 500 to 8,000 cubes 3.65 ms, in turn 3.01).
+		const double wait = res_mixed(form) ? 2.7 : 6.5, work = res_mixed(form) ? 0.012 : 0.07;
+		auto time = [&](int s) { return cost[s] * (wait + work * segWeight[s] / width[s]); };
+		auto later = [&](int a, int b) { return time(a) < time(b); };
+		std::vector<int> heap;
+		for (int s = 0; s < nseg; ++s)
+			if (width[s] < most[s]) heap.push_back(s);
+		std::make_heap(heap.begin(), heap.end(), later);
+		for (; total < ctas && !heap.empty(); ++total)
+		{
+			std::pop_heap(heap.begin(), heap.end(), later);
+			const int s = heap.back();
+			if (++width[s] < most[s])
+				std::push_heap(heap.begin(), heap.end(), later);
+			else
+				heap.pop_back();
+		}
+	}
+	for (int& w : width) w = std::min(w, kResMaxGroup);
 	return width;
 }
 

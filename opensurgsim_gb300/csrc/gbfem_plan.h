@@ -41,9 +41,9 @@ std::vector<int> res_cut(const std::vector<int>& off, int first, int last, int g
 inline int res_chunk_weight(int slots) { return slots + 4; }
 
 // Shares (CTAs) each system gets of `ctas` resident ones. segWeight / segChunks: total chunk weight and chunks of each.
-// local: expected local rows (own and halo) an own row.
+// local: expected local rows (own and halo) an own row; cost: expected iterations of each, up to a factor.
 std::vector<int> res_widths(int form, double local, const std::vector<long long>& segWeight,
-							const std::vector<int>& segChunks, int ctas, int smemBudget);
+							const std::vector<int>& segChunks, const std::vector<double>& cost, int ctas, int smemBudget);
 
 // Plan of the systems whose shares are the chunk ranges between consecutive bounds cut[s], on the SELL
 // matrix (off, rcol: columns as row positions), for `ctas` resident CTAs; cost[s] > 0: expected iterations, which

@@ -70,7 +70,7 @@ int check_plan(int trial)
 			chunks[s] = segChunk[s + 1] - segChunk[s];
 			for (int c = segChunk[s]; c < segChunk[s + 1]; ++c) weight[s] += res_chunk_weight(off[c + 1] - off[c]);
 		}
-		const std::vector<int> width = res_widths(form, 1.7, weight, chunks, ctas, budget);
+		const std::vector<int> width = res_widths(form, 1.7, weight, chunks, std::vector<double>(nseg, 1.0), ctas, budget);
 		std::vector<std::vector<int>> cut(nseg);
 		for (int s = 0; s < nseg; ++s)
 		{
