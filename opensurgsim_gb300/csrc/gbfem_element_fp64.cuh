@@ -167,7 +167,9 @@ __host__ __device__ __forceinline__ void krot_apply(const double (&u)[3][3], con
 
 // The element's results as compute_to defines them, for nodes 0..3 in ascending order of their ids; p, q, uK of
 // nodes 1..3 relative to node 0, g of nodes 1..3. Out: block(a, b, blk) for a >= b, rhs_entry(a, i, v).
-template <typename Out>
+// kPart: the whole element (-1), or a quarter of its results: the right-hand side (0), the blocks of node 3 (1), of
+// node 2 (2), of nodes 0 and 1 (3).
+template <int kPart = -1, typename Out>
 __host__ __device__ __forceinline__ int compute_fp64(const double (&p)[3][3], const double (&q)[3][3],
 													 const double (&uK)[3][3], const double (&uM)[4][3],
 													 const double (&g)[3][3], double lamV, double muV, double cm, bool lumped,
@@ -249,6 +251,7 @@ __host__ __device__ __forceinline__ int compute_fp64(const double (&p)[3][3], co
 #pragma unroll
 	for (int a = 0; a < 3; ++a)
 	{
+		if ((kPart == 1 && a != 2) || (kPart == 2 && a != 1)) continue;
 		const double* ha = h[a + 1];
 		double t[3], L[9];
 #pragma unroll
@@ -273,9 +276,11 @@ __host__ __device__ __forceinline__ int compute_fp64(const double (&p)[3][3], co
 			for (int j = 0; j < 3; ++j)
 				N[a + 1][3 * i + j] = extra ? L[3 * i] * H[j] + L[3 * i + 1] * H[3 + j] + L[3 * i + 2] * H[6 + j] : 0.0;
 	}
+	if constexpr (kPart != 1 && kPart != 2)
 #pragma unroll
-	for (int k = 0; k < 9; ++k) N[0][k] = -(N[1][k] + N[2][k] + N[3][k]);
+		for (int k = 0; k < 9; ++k) N[0][k] = -(N[1][k] + N[2][k] + N[3][k]);
 	// Right-hand side: Krot u~ + N zt with u~ = uK - wr, zt = sum_c h_c x u~_c, and the mass term.
+	if constexpr (kPart <= 0)
 	{
 		double ut[3][3], f[3][3], sum[3];
 #pragma unroll
@@ -302,10 +307,11 @@ __host__ __device__ __forceinline__ int compute_fp64(const double (&p)[3][3], co
 #pragma unroll
 			for (int i = 0; i < 3; ++i) out.rhs_entry(a + 1, i, own * uM[a + 1][i] + (sum[i] + f[a][i]));
 	}
-	if (!out.blocks()) return flags;
+	if (kPart == 0 || !out.blocks()) return flags;
 #pragma unroll
 	for (int a = 0; a < 4; ++a)
 	{
+		if ((kPart == 1 && a != 3) || (kPart == 2 && a != 2) || (kPart == 3 && a > 1)) continue;
 		const double la[3] = {lamV * h[a][0], lamV * h[a][1], lamV * h[a][2]};
 		const double ma[3] = {muV * h[a][0], muV * h[a][1], muV * h[a][2]};
 #pragma unroll

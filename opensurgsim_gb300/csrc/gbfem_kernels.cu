@@ -53,6 +53,11 @@ __global__ void __launch_bounds__(kElemThreads) k_element_fp64(DevBody b, const 
 // arrangement of the same element. Bound by FP64 issue (64 cycles an instruction of a warp on its scheduler,
 // 19 on the SM): about half the instructions of compute_to, 55 us against 116 at 180 tetrahedra (one warp's
 // instructions one after the other), 0.358 ms against 0.769 at 131,905, 0.60 against 1.31 at 225,000.
+// kSplit: four rows of the grid share an element's results (compute_fp64's quarters), each forming what they have in
+// common again, for as many elements as leave schedulers idle: 56 us against 41 up to 1,260 tetrahedra, 56 and 55 at
+// 5,000, 56 and 74 at 8,640.
+constexpr int kElemSplit = 4000;
+template <bool kSplit>
 __global__ void __launch_bounds__(kElemThreads) k_element_corot64(DevBody b, const double* __restrict__ xn,
 																  const double* __restrict__ vn,
 																  const double* __restrict__ xt,
@@ -121,8 +126,18 @@ __global__ void __launch_bounds__(kElemThreads) k_element_corot64(DevBody b, con
 			for (int k = 0; k < 9; ++k) dst[k] = blk[k];
 		}
 	} out{kslots ? kslots + (size_t)e * (kSlots * 9) : nullptr, rhsE + (size_t)e * 12, key};
-	const int fl = elem::compute_fp64(p, q, uK, uM, g, b.rest[13 * (size_t)E + e], b.rest[14 * (size_t)E + e],
-									  b.rest[15 * (size_t)E + e], b.lumped != 0, out);
+	const double lamV = b.rest[13 * (size_t)E + e], muV = b.rest[14 * (size_t)E + e], cm = b.rest[15 * (size_t)E + e];
+	int fl = 0;
+	if constexpr (!kSplit)
+		fl = elem::compute_fp64(p, q, uK, uM, g, lamV, muV, cm, b.lumped != 0, out);
+	else if (blockIdx.y == 0)
+		fl = elem::compute_fp64<0>(p, q, uK, uM, g, lamV, muV, cm, b.lumped != 0, out);
+	else if (blockIdx.y == 1)
+		elem::compute_fp64<1>(p, q, uK, uM, g, lamV, muV, cm, b.lumped != 0, out);
+	else if (blockIdx.y == 2)
+		elem::compute_fp64<2>(p, q, uK, uM, g, lamV, muV, cm, b.lumped != 0, out);
+	else
+		elem::compute_fp64<3>(p, q, uK, uM, g, lamV, muV, cm, b.lumped != 0, out);
 	if (fl & 1) atomicAdd(&counters[1], 1);
 	if (fl & 2) atomicAdd(&counters[0], 1);
 }
@@ -1099,8 +1114,12 @@ void launch_element_fp64(const DevBody& b, const double* xn, const double* vn, c
 	else if (linear)
 		k_element_fp64<false, true><<<nb, kElemThreads, 0, s>>>(b, xn, vn, xt, vt, dt, alpha, beta, kslots, rhsE,
 																 nullptr, nullptr, counters);
+	else if (kslots && b.E <= kElemSplit)
+		k_element_corot64<true><<<dim3(nb, 4), kElemThreads, 0, s>>>(b, xn, vn, xt, vt, dt, 1.0 / dt, alpha, beta, kslots, rhsE,
+																	 counters);
 	else
-		k_element_corot64<<<nb, kElemThreads, 0, s>>>(b, xn, vn, xt, vt, dt, 1.0 / dt, alpha, beta, kslots, rhsE, counters);
+		k_element_corot64<false><<<nb, kElemThreads, 0, s>>>(b, xn, vn, xt, vt, dt, 1.0 / dt, alpha, beta, kslots, rhsE,
+															 counters);
 }
 
 int launch_element_f32(const DevBody& b, const double* xn, const double* vn, const double* xt, const double* vt,
