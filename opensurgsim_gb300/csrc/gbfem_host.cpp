@@ -872,7 +872,7 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 	// schedule's result bit for bit; batches that had the two-phase schedule keep that too. Larger systems take
 	// the rows of a share from one compact box, as FP64 systems do: the halo is a half to a third
 	// (50,653 nodes on 152 CTAs: 4.1 local rows an own row in node order, 1.8 in boxes; a batch of 687,000
-	// nodes does not fit in node order at all, and its solve takes 5.7 ms in boxes, 15.4 two-phase).
+	// nodes does not fit in node order at all, and its solve takes 5.0 ms in boxes, 15.4 two-phase).
 	SellOrder so;
 	int chunks = 0;
 	for (int sg = 0; sg < nseg; ++sg) chunks += (h->segNode[sg + 1] - h->segNode[sg] + 31) / 32;

@@ -21,12 +21,13 @@
 // needs), groups side by side and, when they outnumber the SMs, one after the other.
 //
 // Solve times, before (gbfem_pcg.cu's, of one launch an iteration or persistent) and here: FP64 80 nodes 2.9
-// and 0.45 ms, 1,331 nodes 3.3 and 0.58, 29,184 nodes 4.1 and 1.33, 24 meshes 10.4 and 3.3; mixed 1,331
-// nodes 1.40 and 0.40, 18,081 nodes 1.93 and 0.53, 270,641 nodes (410 iterations) 18.3 and 15.3, 64 meshes 15.7
-// and 5.7; 12 compliance columns of 1,331 nodes 47 and 0.94; a caller's matrix of 17,280 rows 2.98 and 0.50.
-// What bounds them: the two waits of an FP64 iteration (2 x 1.6 us of 5.6) and the one of a mixed
-// iteration (1.6 of 4.8), the FP64 rate (64 cycles an instruction of a warp) in FP64 products, and the L2
-// reads of what does not fit in shared memory in large systems.
+// and 0.34 ms, 1,331 nodes 3.3 and 0.49, 29,184 nodes 4.1 and 1.18, 24 meshes 10.4 and 3.0; mixed 1,331
+// nodes 1.40 and 0.23, 18,081 nodes 1.93 and 0.38, 270,641 nodes (410 iterations) 18.3 and 12.5, 64 meshes 15.7
+// and 5.0; 12 compliance columns of 1,331 nodes 47 and 0.94; a caller's matrix of 17,280 rows 2.98 and 0.46.
+// What bounds them: the waits of an iteration (a sum over CTAs takes 0.5 us in a cluster, 1.2 to 1.8 us through L2;
+// FP64 has two an iteration of 4.5 to 15 us, mixed one of 2.7 to 4.5), the FP64 rate (64 cycles an instruction
+// of a warp) in FP64 products and sums, and the L2 and HBM reads of what does not fit in shared memory in large
+// systems.
 
 #include <cfloat>
 #include <cstdint>
@@ -239,11 +240,13 @@ struct Share
 	const unsigned char *val, *col;  // the same in global memory
 };
 
-// Warps that share the product: an FP64 instruction takes 64 cycles of a scheduler and 19 of the SM, so four
-// warps nearly saturate it, and every piece more a chunk is cut into costs its rows an FP64 add.
+// Warps that share the product: an FP64 instruction takes 64 cycles of a scheduler and 19 of the SM, so few warps
+// saturate it, and every piece more a chunk is cut into costs its rows an FP64 add (solves of 1,331 nodes, one chunk a
+// share: 0.508 ms with 4 warps, 0.485 with 7, 0.494 with 10; of 4,913, two to four chunks: 0.667 with 4 and 8, 0.623
+// with 7 and 10).
 __device__ __forceinline__ int product_warps(int nCh)
 {
-	return nCh <= 2 ? 4 : (nCh <= 4 ? 8 : kResRowWarps);
+	return nCh <= 2 ? 7 : (nCh <= 4 ? 10 : kResRowWarps);
 }
 __device__ __forceinline__ int part_first(int w, int n, int nw) { return w >= nw ? n : w * n / nw; }
 

@@ -112,7 +112,7 @@ int check_plan(int trial)
 				CHECK(keptAt(0) == 0 && keptAt(L.nCh) == kept && L.pieces + 4 * (L.nCh + 1) <= L.halo);
 				continue;
 			}
-			const int nw = (int)std::min<long long>(slots, L.nCh <= 2 ? 4 : (L.nCh <= 4 ? 8 : kResRowWarps));
+			const int nw = (int)std::min<long long>(slots, L.nCh <= 2 ? 7 : (L.nCh <= 4 ? 10 : kResRowWarps));
 			auto first = [&](int w) { return w >= nw ? (int)slots : (int)(w * slots / nw); };
 			auto keptFirst = [&](int w) { return w >= nw ? kept : w * kept / nw; };
 			auto at = [&](int c) { return off[p.c0 + c] - off[p.c0]; };
