@@ -54,17 +54,34 @@ struct DevBuf
 	}
 };
 
-// Dynamic shared memory the resident solve's kernel may use, raised as needed (once per process and form).
+// Dynamic shared memory limits of kernel forms: attributes of a kernel on a device, shared by the process. Only ever
+// raised, so a launch sized for one handle never breaks another's.
+struct SmemLimits
+{
+	std::mutex mu;
+	std::map<std::pair<int, int>, size_t> raised;  // by device and form; 48 KB without an entry
+	cudaError_t raise(size_t bytes, int form, cudaError_t (*set)(int, int))
+	{
+		int device = 0;
+		const cudaError_t got = cudaGetDevice(&device);
+		if (got != cudaSuccess) return got;
+		std::lock_guard<std::mutex> lock(mu);
+		size_t& limit = raised.emplace(std::make_pair(device, form), 48 * 1024).first->second;
+		if (bytes <= limit) return cudaSuccess;
+		const cudaError_t e = set(form, (int)bytes);
+		if (e == cudaSuccess) limit = bytes;
+		return e;
+	}
+};
 cudaError_t raise_res_smem_limit(size_t bytes, int form)
 {
-	static std::mutex mu;
-	static size_t current[kResForms] = {};
-	std::lock_guard<std::mutex> lock(mu);
-	size_t& c = current[form];
-	if (bytes <= std::max<size_t>(c, 48 * 1024)) return cudaSuccess;
-	const cudaError_t e = res_set_max_dynamic_smem(form, (int)bytes);
-	if (e == cudaSuccess) c = bytes;
-	return e;
+	static SmemLimits limits;
+	return limits.raise(bytes, form, res_set_max_dynamic_smem);
+}
+cudaError_t raise_pcg_smem_limit(size_t bytes, int form)
+{
+	static SmemLimits limits;
+	return limits.raise(bytes, form, pcg_set_max_dynamic_smem);
 }
 
 // Shared memory of a resident CTA: one CTA an SM, less its reserved 1 KB and the kernel's static part.
@@ -531,19 +548,6 @@ gbfem_status fail(gbfem_handle h, gbfem_status st, const std::string& msg)
 			return fail(h, e_ == cudaErrorMemoryAllocation ? GBFEM_OUT_OF_MEMORY : GBFEM_CUDA_ERROR,     \
 						std::string(#call) + ": " + cudaGetErrorString(e_));                            \
 	} while (0)
-
-// The persistent solve's dynamic shared memory limit is a process-wide attribute of the kernel:
-// only ever raised, so a launch sized for one handle never breaks another's.
-cudaError_t raise_pcg_smem_limit(size_t bytes, int form)
-{
-	static std::mutex mu;
-	static size_t current[3] = {48 * 1024, 48 * 1024, 48 * 1024};
-	std::lock_guard<std::mutex> lock(mu);
-	if (bytes <= current[form]) return cudaSuccess;
-	const cudaError_t e = pcg_set_max_dynamic_smem(form, (int)bytes);
-	if (e == cudaSuccess) current[form] = bytes;
-	return e;
-}
 
 // Grid of the persistent solve for `cps` CTAs per SM and the handle's refresh weight rw:
 // G = min(cps * SMs, chunks); the largest share of a CTA in chunks (its shared-memory partials) is

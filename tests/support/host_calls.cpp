@@ -1,0 +1,283 @@
+// The host side of the C entry points (gbfem_host.cpp, gbfem_plan.cpp) on a stand-in for the CUDA runtime that
+// lives in host memory: two devices, allocations that can be made to fail, solves that can be made to report that
+// a wait ran out. Kernels do nothing. Runs the case named on the command line and prints "ok" or what went wrong.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <functional>
+#include <map>
+#include <new>
+#include <string>
+#include <vector>
+
+#include "../../include/gbfem.h"
+#include "gbfem_pcg.h"
+#include "gbfem_res.h"
+
+#define CHECK(x)                                              \
+	do                                                        \
+		if (!(x))                                             \
+		{                                                     \
+			std::printf("line %d: %s\n", __LINE__, #x);       \
+			std::exit(1);                                     \
+		}                                                     \
+	while (0)
+
+// ---- the stand-in -------------------------------------------------------------------------------------------------
+namespace fake {
+
+int device = 0;                          // current device
+std::map<std::pair<int, int>, int> res;  // dynamic shared memory limit of a resident form on a device
+std::map<std::pair<int, int>, int> pcg;  // and of a persistent one
+std::map<void*, size_t> blocks;          // device memory
+long long allocations = 0, failAt = -1;  // the allocation that fails, counted from zero
+int solves = 0;
+bool giveUp = false;                     // whether solves report a wait that ran out
+bool capturing = false;
+std::function<void()> solve;             // repeated by a graph launch
+
+int limit(const std::map<std::pair<int, int>, int>& m, int form)
+{
+	const auto it = m.find({device, form});
+	return it == m.end() ? 48 * 1024 : it->second;
+}
+
+}  // namespace fake
+
+extern "C" {
+
+cudaError_t cudaGetDevice(int* d)
+{
+	*d = fake::device;
+	return cudaSuccess;
+}
+cudaError_t cudaSetDevice(int d)
+{
+	if (d < 0 || d > 1) return cudaErrorInvalidDevice;
+	fake::device = d;
+	return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int)
+{
+	*v = a == cudaDevAttrMultiProcessorCount ? 152 : (a == cudaDevAttrMaxSharedMemoryPerMultiprocessor ? 228 * 1024 : 0);
+	return cudaSuccess;
+}
+cudaError_t cudaMalloc(void** p, size_t n)
+{
+	if (fake::allocations++ == fake::failAt) return cudaErrorMemoryAllocation;
+	*p = std::calloc(n, 1);
+	fake::blocks[*p] = n;
+	return cudaSuccess;
+}
+cudaError_t cudaFree(void* p)
+{
+	CHECK(fake::blocks.erase(p) == 1);
+	std::free(p);
+	return cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned)
+{
+	*p = std::calloc(n, 1);
+	return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void* p)
+{
+	std::free(p);
+	return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind)
+{
+	CHECK(n == 0 || (d && s));
+	if (n && !fake::capturing) std::memmove(d, s, n);
+	return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t)
+{
+	return cudaMemcpy(d, s, n, k);
+}
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t)
+{
+	CHECK(n == 0 || d);
+	if (n && !fake::capturing) std::memset(d, v, n);
+	return cudaSuccess;
+}
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode)
+{
+	fake::capturing = true;
+	return cudaSuccess;
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t*)
+{
+	fake::capturing = false;
+	return cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t)
+{
+	fake::solve();
+	return cudaSuccess;
+}
+const char* cudaGetErrorString(cudaError_t) { return "stand-in error"; }
+
+}  // extern "C"
+
+namespace gbfem {
+
+cudaError_t res_set_max_dynamic_smem(int form, int bytes)
+{
+	fake::res[{fake::device, form}] = bytes;
+	return cudaSuccess;
+}
+bool res_cluster_fits(int, int, size_t) { return false; }
+cudaError_t res_launch(int form, int, size_t smem, const ResArgs& a, cudaStream_t)
+{
+	if ((long long)smem > fake::limit(fake::res, form)) return cudaErrorInvalidValue;
+	CHECK(a.parts && a.tasks && a.lcol && a.off && a.perm && a.ctl && a.seg && a.err && a.b && a.x && a.val && a.invdiag);
+	CHECK(a.mail && a.rowWords);
+	if (res_mixed(form)) CHECK(a.xhl && a.r64 && a.chunkWarp && a.chunkList);
+	auto run = [a] {
+		CHECK(*a.err == 0);  // a flag left set would end this launch's waits at once
+		++fake::solves;
+		for (int t = 0; t < a.nTasks; ++t)
+		{
+			SegCtl& c = a.seg[a.parts[a.tasks[t].x].seg + (size_t)a.tasks[t].y * a.segStride];
+			c = SegCtl{};
+			c.bb = 1.0;
+			c.converged = 1;
+			c.iter = 3;
+		}
+		if (fake::giveUp) *a.err = 1;
+	};
+	if (!fake::capturing) run();
+	fake::solve = run;
+	return cudaSuccess;
+}
+cudaError_t pcg_set_max_dynamic_smem(int form, int bytes)
+{
+	fake::pcg[{fake::device, form}] = bytes;
+	return cudaSuccess;
+}
+cudaError_t pcg_occupancy(int, int* n, size_t)
+{
+	*n = 4;
+	return cudaSuccess;
+}
+cudaError_t pcg_launch(int form, const cudaLaunchConfig_t& cfg, const PcgArgs&)
+{
+	return (long long)cfg.dynamicSmemBytes > fake::limit(fake::pcg, form) ? cudaErrorInvalidValue : cudaSuccess;
+}
+void launch_step_accumulate(const SegCtl*, int nseg, const int*, const int* err, double* acc, cudaStream_t)
+{
+	fake::solve = [=, before = fake::solve] {
+		before();
+		if (*err) acc[4 * nseg + 1] = 1.0;
+	};
+}
+
+}  // namespace gbfem
+
+// ---- the cases ----------------------------------------------------------------------------------------------------
+namespace {
+
+// a x b x c unit cubes of six tetrahedra, the first node fixed, `spare` nodes of no element after the others.
+struct Grid
+{
+	std::vector<double> X, Ey, Nu, Rho;
+	std::vector<int32_t> T, bc{0, 1, 2};
+	gbfem_mesh_desc desc{};
+	Grid(int a, int b, int c, int spare = 0, double at = 0.0)
+	{
+		auto id = [&](int i, int j, int k) { return (i * (b + 1) + j) * (c + 1) + k; };
+		for (int i = 0; i <= a; ++i)
+			for (int j = 0; j <= b; ++j)
+				for (int k = 0; k <= c; ++k)
+					for (double v : {0.01 * i, 0.01 * j, 0.01 * k}) X.push_back(v);
+		X.insert(X.end(), 3 * spare, at);
+		const int order[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
+		for (int i = 0; i < a; ++i)
+			for (int j = 0; j < b; ++j)
+				for (int k = 0; k < c; ++k)
+					for (int o = 0; o < 6; ++o)
+					{
+						int p[3] = {i, j, k};
+						int t[4] = {id(p[0], p[1], p[2])};
+						for (int s = 0; s < 3; ++s)
+						{
+							++p[order[o][s]];
+							t[s + 1] = id(p[0], p[1], p[2]);
+						}
+						if (o == 1 || o == 2 || o == 5) std::swap(t[2], t[3]);  // odd orders: a positive volume
+						T.insert(T.end(), t, t + 4);
+					}
+		const size_t E = T.size() / 4;
+		Ey.assign(E, 1e5);
+		Nu.assign(E, 0.4);
+		Rho.assign(E, 1000.0);
+		desc = gbfem_mesh_desc{(int32_t)(X.size() / 3), X.data(), (int32_t)E, T.data(), Ey.data(), Nu.data(), Rho.data(),
+							   (int32_t)bc.size(), bc.data()};
+	}
+};
+
+gbfem_params params(int precision, int device)
+{
+	gbfem_params p;
+	gbfem_params_default(&p);
+	p.precision = precision;
+	p.device = device;
+	return p;
+}
+
+gbfem_handle create(const Grid& g, int precision, int device = 0)
+{
+	const gbfem_params p = params(precision, device);
+	gbfem_handle h = nullptr;
+	CHECK(gbfem_create(&g.desc, &p, &h) == GBFEM_OK);
+	return h;
+}
+
+// Bodies, compliance and caller's matrices on a second device after the same on the first.
+void two_devices()
+{
+	const Grid g(10, 10, 10);
+	for (int precision : {GBFEM_PRECISION_FP64, GBFEM_PRECISION_MIXED})
+		for (int device = 0; device < 2; ++device)
+		{
+			gbfem_handle h = create(g, precision, device);
+			CHECK(gbfem_step(h, 1e-3, 1, 0) == GBFEM_OK);
+			std::vector<double> b(3 * g.X.size(), 1.0), x(b.size());
+			CHECK(gbfem_apply_compliance(h, 3, b.data(), x.data(), 0, nullptr) == GBFEM_OK);
+			gbfem_destroy(h);
+		}
+	const int n = 4000;
+	std::vector<int32_t> ptr{0}, row;
+	std::vector<double> val;
+	for (int c = 0; c < n; ++c)
+	{
+		row.push_back(c);
+		val.push_back(4.0);
+		if (c + 1 < n) row.push_back(c + 1), val.push_back(-1.0);
+		ptr.push_back((int32_t)row.size());
+	}
+	for (int device = 0; device < 2; ++device)
+	{
+		gbfem_cg cg = nullptr;
+		CHECK(gbfem_cg_create(n, ptr.data(), row.data(), val.data(), device, &cg) == GBFEM_OK);
+		std::vector<double> b(n, 1.0), x(n);
+		CHECK(gbfem_cg_solve(cg, b.data(), x.data(), nullptr, nullptr) == GBFEM_OK);
+		gbfem_cg_destroy(cg);
+	}
+}
+
+}  // namespace
+
+int main(int argc, char** argv)
+{
+	const std::map<std::string, void (*)()> cases = {
+		{"two_devices", two_devices},
+	};
+	const auto it = cases.find(argc > 1 ? argv[1] : "");
+	CHECK(it != cases.end());
+	it->second();
+	CHECK(fake::blocks.empty());
+	std::printf("ok\n");
+	return 0;
+}
