@@ -36,9 +36,13 @@ struct DevBuf
 	cudaError_t alloc(size_t count)
 	{
 		free();
-		n = count;
 		if (count == 0) return cudaSuccess;
-		return cudaMalloc(&p, count * sizeof(T));
+		const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+		if (e == cudaSuccess)
+			n = count;  // a buffer that was not had stays empty: the next call asks for it again
+		else
+			p = nullptr;
+		return e;
 	}
 	cudaError_t upload(const T* src, size_t count, cudaStream_t s)
 	{
@@ -1190,7 +1194,7 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 // Lazily built maps for exporting the full (non-mirrored) system in CSC order.
 gbfem_status ensure_system_maps(gbfem_handle h)
 {
-	if (h->d_sptr.p) return GBFEM_OK;
+	if (h->d_f.p) return GBFEM_OK;
 	const int E = h->E;
 	const int64_t nnz = h->nnz;
 	std::vector<int> slot((size_t)E * 144);
@@ -1893,7 +1897,7 @@ gbfem_status step_once(gbfem_handle h, double dt, uint32_t flags)
 	double* vt = h->d_v.p;
 	if (newtonMax > 1)
 	{
-		if (!h->d_xt.p)
+		if (!h->d_dvPrev.p)
 		{
 			GB_CUDA(h, h->d_xt.alloc(h->n));
 			GB_CUDA(h, h->d_vt.alloc(h->n));
@@ -2303,12 +2307,9 @@ gbfem_status compliance_resident(gbfem_handle h, ResDevice& d, int ncols, const 
 	const int n = h->n, most = std::min(d.maxRhs, ncols);
 	const size_t mailStride = d.plan.mailWords, rowStride = (size_t)res_row_words(d.plan.form) * h->nrows;
 	GB_CUDA(h, h->colLink.reserve(mailStride * most, rowStride * most, s));
-	if (h->d_colSeg.n < (size_t)most)
-	{
-		GB_CUDA(h, h->d_colB.alloc((size_t)n * most));
-		GB_CUDA(h, h->d_colX.alloc((size_t)n * most));
-		GB_CUDA(h, h->d_colSeg.alloc(most));
-	}
+	if (h->d_colB.n < (size_t)n * most) GB_CUDA(h, h->d_colB.alloc((size_t)n * most));
+	if (h->d_colX.n < (size_t)n * most) GB_CUDA(h, h->d_colX.alloc((size_t)n * most));
+	if (h->d_colSeg.n < (size_t)most) GB_CUDA(h, h->d_colSeg.alloc(most));
 	if (!h->d_colErr.p)
 	{
 		GB_CUDA(h, h->d_colErr.alloc(1));
@@ -2392,7 +2393,7 @@ gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double*
 			return fail(h, GBFEM_OUT_OF_MEMORY, "gbfem_apply_compliance: out of host memory");
 		}
 	}
-	if (!columns && !h->d_mcgVec.p)
+	if (!columns && !h->h_mcgCtl)
 	{
 		GB_CUDA(h, h->d_mcgVec.alloc(6 * n8));
 		GB_CUDA(h, h->d_mcgPart.alloc(2 * (size_t)kMcgCols * L.vecGrid));
@@ -2403,7 +2404,7 @@ gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double*
 	const DevBody body = h->body();
 	if (warp)
 	{
-		if (!h->d_Qe.p)
+		if (!h->d_xprev.p)
 		{
 			GB_CUDA(h, h->d_Qe.alloc(4 * (size_t)h->E));
 			GB_CUDA(h, h->d_Wn.alloc(9 * (size_t)N));
@@ -2600,7 +2601,7 @@ gbfem_status gbfem_adjoint_step(gbfem_handle h, double dt, const double* x, cons
 	cudaStream_t s = h->stream;
 	const DevBody body = h->body();
 	const int n = h->n;
-	if (!h->d_mu.p)
+	if (!h->d_gv.p)
 	{
 		GB_CUDA(h, h->d_mu.alloc(n));
 		GB_CUDA(h, h->d_adjG.alloc(n));
@@ -2666,7 +2667,7 @@ namespace {
 
 gbfem_status ensure_adjoint_buffers(gbfem_handle h)
 {
-	if (h->d_mu.p) return GBFEM_OK;
+	if (h->d_gv.p) return GBFEM_OK;
 	GB_CUDA(h, h->d_mu.alloc(h->n));
 	GB_CUDA(h, h->d_adjG.alloc(h->n));
 	GB_CUDA(h, h->d_gx.alloc(12 * (size_t)h->E));
@@ -3146,7 +3147,7 @@ gbfem_status gbfem_set_velocities(gbfem_handle h, int32_t count, const int32_t* 
 		if (dofs[i] < 0 || dofs[i] >= h->n) return fail(h, GBFEM_INVALID_ARG, "dof out of range");
 	if (count == 0) return GBFEM_OK;
 	GB_CUDA(h, cudaSetDevice(h->device));
-	if (h->d_idx.n < (size_t)count)
+	if (h->d_vals.n < (size_t)count)
 	{
 		GB_CUDA(h, h->d_idx.alloc(count));
 		GB_CUDA(h, h->d_vals.alloc(count));

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/gbfem.h"
+#include "gbfem_internal.h"
 #include "gbfem_pcg.h"
 #include "gbfem_res.h"
 
@@ -111,6 +112,11 @@ cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t*)
 	fake::capturing = false;
 	return cudaSuccess;
 }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long)
+{
+	*e = reinterpret_cast<cudaGraphExec_t>(&fake::solve);
+	return cudaSuccess;
+}
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t)
 {
 	fake::solve();
@@ -171,6 +177,31 @@ void launch_step_accumulate(const SegCtl*, int nseg, const int*, const int* err,
 		before();
 		if (*err) acc[4 * nseg + 1] = 1.0;
 	};
+}
+
+void launch_mcg_init(int, int, const double* B, const uint8_t*, const double*, const float*, double*, double*, double*,
+					 double*, McgCtl* ctl, double* part, double, int, const Launch&)
+{
+	CHECK(B && ctl && part);
+	ctl->allDone = 1;
+	for (int& c : ctl->converged) c = 1;
+}
+void launch_node_rotation(const DevBody&, const double* Qe, double* Wn, cudaStream_t) { CHECK(Qe && Wn); }
+void launch_element_adjoint(const DevBody&, const double*, const double*, const double* mu, const double* dv, double, double,
+							double, double* gx, double* gv, double*, double*, cudaStream_t, bool)
+{
+	CHECK(mu && dv && gx && gv);
+}
+void launch_scatter_values(int, const int* idx, const double* v, double*, cudaStream_t) { CHECK(idx && v); }
+void launch_state_update(int, const double*, double* dvPrev, const double* xt, double*, double*, double, int newton, CgCtl*,
+						 double*, const Launch&)
+{
+	CHECK(xt && (!newton || dvPrev));
+}
+void launch_assemble_full_csc(int, const int* a, const int* b, const int* c, const int* d, const double* k, const double* m,
+							  const uint8_t*, double, double, double* S, cudaStream_t)
+{
+	CHECK(a && b && c && d && k && m && S);
 }
 
 }  // namespace gbfem
@@ -267,12 +298,93 @@ void two_devices()
 	}
 }
 
+// f() with each of its allocations failing in turn, and again once memory is there; then without a failure.
+template <typename F>
+void every_allocation(F f)
+{
+	for (int k = 0;; ++k)
+	{
+		fake::failAt = fake::allocations + k;
+		const gbfem_status st = f();
+		const bool failed = fake::allocations > fake::failAt;
+		fake::failAt = -1;
+		if (!failed)
+		{
+			CHECK(st == GBFEM_OK);
+			return;
+		}
+		CHECK(st == GBFEM_OUT_OF_MEMORY);
+		if (k % 2 == 0) continue;  // two failures in a row as well as one
+		CHECK(f() == GBFEM_OK);
+	}
+}
+
+// Calls whose buffers cannot be had report it and can be made again.
+void failed_allocations()
+{
+	const Grid g(6, 6, 6);
+	const size_t n = g.X.size();
+	std::vector<double> b(200 * n, 1.0), x(200 * n), y(n), z(n), w(n);
+	std::vector<int32_t> dofs(n);
+	for (int precision : {GBFEM_PRECISION_FP64, GBFEM_PRECISION_MIXED})
+	{
+		gbfem_params p = params(precision, 0);
+		p.newton_max_iterations = 2;
+		gbfem_handle h = nullptr;
+		every_allocation([&] {
+			if (h) gbfem_destroy(h);
+			h = nullptr;
+			return gbfem_create(&g.desc, &p, &h);
+		});
+		every_allocation([&] { return gbfem_step(h, 1e-3, 1, precision == GBFEM_PRECISION_FP64 ? GBFEM_STEP_KEEP_SYSTEM : 0); });
+		for (int columns : {3, 200, 3, 40})
+			every_allocation([&] {
+				return gbfem_apply_compliance(h, columns, b.data(), x.data(), GBFEM_COMPLIANCE_WARPING, nullptr);
+			});
+		every_allocation([&] { return gbfem_set_velocities(h, 1, dofs.data(), b.data()); });
+		every_allocation([&] { return gbfem_set_velocities(h, (int)n, dofs.data(), b.data()); });
+		every_allocation([&] {
+			return gbfem_adjoint_step(h, 1e-3, b.data(), b.data(), b.data(), b.data(), b.data(), y.data(), z.data(), w.data(),
+									  nullptr, 0);
+		});
+		gbfem_destroy(h);
+		// A batch: columns eight at a time; rollouts.
+		const gbfem_mesh_desc two[2] = {g.desc, g.desc};
+		p.newton_max_iterations = 1;
+		CHECK(gbfem_batch_create(2, two, &p, &h) == GBFEM_OK);
+		CHECK(gbfem_step(h, 1e-3, 1, 0) == GBFEM_OK);
+		std::vector<double> lx(2 * n), lv(2 * n), x0(2 * n), v0(2 * n);
+		every_allocation([&] {
+			return gbfem_apply_compliance(h, 2, b.data(), x.data(), GBFEM_COMPLIANCE_WARPING, nullptr);
+		});
+		for (int steps : {2, 6})
+		{
+			every_allocation([&] {
+				return gbfem_rollout_forward(h, 1e-3, steps, steps / 2, b.data(), b.data(), x0.data(), v0.data());
+			});
+			every_allocation([&] {
+				return gbfem_rollout_backward(h, b.data(), b.data(), lx.data(), lv.data(), nullptr, nullptr);
+			});
+		}
+		gbfem_destroy(h);
+	}
+	gbfem_cg cg = nullptr;
+	const std::vector<int32_t> ptr{0, 1, 2}, row{0, 1};
+	every_allocation([&] {
+		if (cg) gbfem_cg_destroy(cg);
+		cg = nullptr;
+		return gbfem_cg_create(2, ptr.data(), row.data(), b.data(), 0, &cg);
+	});
+	gbfem_cg_destroy(cg);
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
 {
 	const std::map<std::string, void (*)()> cases = {
 		{"two_devices", two_devices},
+		{"failed_allocations", failed_allocations},
 	};
 	const auto it = cases.find(argc > 1 ? argv[1] : "");
 	CHECK(it != cases.end());
