@@ -2280,17 +2280,29 @@ gbfem_status compliance_plan(gbfem_handle h, int ncols, ResDevice** out)
 				for (int& r : rcol) r = iperm[r];  // on padding slots any row of the system will do: their values are zero
 			}
 			ResPlan plan = res_plan(form, {res_cut(off, 0, h->nchunks, c.g)}, off, rcol, {1.0}, h->smCount, h->resBudget);
-			ResDevice d;
 			if (plan.ok)
 			{
 				// Columns a launch takes: four waves, at most 256 MB of exchanged rows.
 				const int waves = 4 * (h->smCount / c.g);
 				const int room = (int)std::max<int64_t>(1, ((int64_t)256 << 20) / (48LL * h->nrows));
-				const cudaError_t e = d.upload(std::move(plan), off, h->resBudget, std::min(waves, room), h->stream);
-				if (e != cudaSuccess) d.free();
+				have = h->colPlans.emplace(c.g, ResDevice()).first;
+				cudaError_t e = cudaErrorMemoryAllocation;
+				try
+				{
+					e = have->second.upload(std::move(plan), off, h->resBudget, std::min(waves, room), h->stream);
+				}
+				catch (const std::bad_alloc&)
+				{
+				}
+				if (e != cudaSuccess)
+				{
+					have->second.free();
+					h->colPlans.erase(have);
+				}
 				GB_CUDA(h, e);
 			}
-			have = h->colPlans.emplace(c.g, std::move(d)).first;
+			else
+				have = h->colPlans.emplace(c.g, ResDevice()).first;
 		}
 		if (!have->second.plan.ok) continue;
 		*out = &have->second;
@@ -2364,12 +2376,9 @@ gbfem_status compliance_resident(gbfem_handle h, ResDevice& d, int ncols, const 
 	return GBFEM_OK;
 }
 
-}  // namespace
-
-gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double* b, double* x, uint32_t flags,
-									int32_t* iterations)
+gbfem_status apply_compliance(gbfem_handle h, int32_t ncols, const double* b, double* x, uint32_t flags,
+							  int32_t* iterations)
 {
-	if (!h) return GBFEM_INVALID_ARG;
 	if (ncols < 0 || (ncols > 0 && (!b || !x))) return fail(h, GBFEM_INVALID_ARG, "gbfem_apply_compliance: bad arrays");
 	if (!h->systemReady) return fail(h, GBFEM_INVALID_ARG, "gbfem_apply_compliance: no step has assembled a system yet");
 	const bool warp = (flags & GBFEM_COMPLIANCE_WARPING) != 0;
@@ -2383,15 +2392,8 @@ gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double*
 	ResDevice* columns = nullptr;
 	if (ncols > 0)
 	{
-		try
-		{
-			const gbfem_status st = compliance_plan(h, ncols, &columns);
-			if (st != GBFEM_OK) return st;
-		}
-		catch (const std::bad_alloc&)
-		{
-			return fail(h, GBFEM_OUT_OF_MEMORY, "gbfem_apply_compliance: out of host memory");
-		}
+		const gbfem_status st = compliance_plan(h, ncols, &columns);
+		if (st != GBFEM_OK) return st;
 	}
 	if (!columns && !h->h_mcgCtl)
 	{
@@ -2469,6 +2471,22 @@ gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double*
 	}
 	if (iterations) *iterations = totalIt;
 	return allConverged ? GBFEM_OK : fail(h, GBFEM_CG_MAXITER, "a compliance column did not converge");
+}
+
+}  // namespace
+
+gbfem_status gbfem_apply_compliance(gbfem_handle h, int32_t ncols, const double* b, double* x, uint32_t flags,
+									int32_t* iterations)
+{
+	if (!h) return GBFEM_INVALID_ARG;
+	try
+	{
+		return apply_compliance(h, ncols, b, x, flags, iterations);
+	}
+	catch (const std::bad_alloc&)
+	{
+		return fail(h, GBFEM_OUT_OF_MEMORY, "gbfem_apply_compliance: out of host memory");
+	}
 }
 
 gbfem_status gbfem_get_tuning(gbfem_handle h, int32_t* elems_per_block, int32_t* ctas_per_sm, int32_t* refresh_weight,

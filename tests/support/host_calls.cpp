@@ -32,6 +32,7 @@ std::map<std::pair<int, int>, int> res;  // dynamic shared memory limit of a res
 std::map<std::pair<int, int>, int> pcg;  // and of a persistent one
 std::map<void*, size_t> blocks;          // device memory
 long long allocations = 0, failAt = -1;  // the allocation that fails, counted from zero
+long long news = 0, newFails = -1;       // the same of the host's memory, which `new` gives
 int solves = 0;
 bool giveUp = false;                     // whether solves report a wait that ran out
 bool capturing = false;
@@ -44,6 +45,16 @@ int limit(const std::map<std::pair<int, int>, int>& m, int form)
 }
 
 }  // namespace fake
+
+void* operator new(size_t n)
+{
+	if (fake::news++ == fake::newFails) throw std::bad_alloc();
+	if (void* p = std::malloc(n ? n : 1)) return p;
+	throw std::bad_alloc();
+}
+void* operator new(size_t n, const std::nothrow_t&) noexcept { return std::malloc(n ? n : 1); }
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 extern "C" {
 
@@ -67,7 +78,11 @@ cudaError_t cudaMalloc(void** p, size_t n)
 {
 	if (fake::allocations++ == fake::failAt) return cudaErrorMemoryAllocation;
 	*p = std::calloc(n, 1);
+	const long long fails = fake::newFails, news = fake::news;
+	fake::newFails = -1;  // the record below is not the caller's
 	fake::blocks[*p] = n;
+	fake::newFails = fails;
+	fake::news = news;
 	return cudaSuccess;
 }
 cudaError_t cudaFree(void* p)
@@ -154,7 +169,7 @@ cudaError_t res_launch(int form, int, size_t smem, const ResArgs& a, cudaStream_
 		if (fake::giveUp) *a.err = 1;
 	};
 	if (!fake::capturing) run();
-	fake::solve = run;
+	if (fake::capturing) fake::solve = run;
 	return cudaSuccess;
 }
 cudaError_t pcg_set_max_dynamic_smem(int form, int bytes)
@@ -378,6 +393,33 @@ void failed_allocations()
 	gbfem_cg_destroy(cg);
 }
 
+// Compliance calls that run out of host memory say so.
+void failed_host_memory()
+{
+	const Grid g(6, 6, 6);
+	const size_t n = g.X.size();
+	const gbfem_params p = params(GBFEM_PRECISION_FP64, 0);
+	const gbfem_mesh_desc two[2] = {g.desc, g.desc};
+	std::vector<double> b(80 * n, 1.0), x(80 * n);
+	for (int batch = 0; batch < 2; ++batch)
+	{
+		gbfem_handle h = nullptr;
+		CHECK((batch ? gbfem_batch_create(2, two, &p, &h) : gbfem_create(&g.desc, &p, &h)) == GBFEM_OK);
+		CHECK(gbfem_step(h, 1e-3, 1, 0) == GBFEM_OK);
+		for (int columns : {2, 40})
+			for (int k = 0;; ++k)
+			{
+				fake::newFails = fake::news + k;
+				const gbfem_status st = gbfem_apply_compliance(h, columns, b.data(), x.data(), 0, nullptr);
+				const bool failed = fake::news > fake::newFails;
+				fake::newFails = -1;
+				CHECK(st == (failed ? GBFEM_OUT_OF_MEMORY : GBFEM_OK));
+				if (!failed) break;
+			}
+		gbfem_destroy(h);
+	}
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -385,6 +427,7 @@ int main(int argc, char** argv)
 	const std::map<std::string, void (*)()> cases = {
 		{"two_devices", two_devices},
 		{"failed_allocations", failed_allocations},
+		{"failed_host_memory", failed_host_memory},
 	};
 	const auto it = cases.find(argc > 1 ? argv[1] : "");
 	CHECK(it != cases.end());
