@@ -1472,6 +1472,16 @@ gbfem_status enqueue_mixed(gbfem_handle h, const double* b, double* x, int maxIt
 	return GBFEM_OK;
 }
 
+// Reports a solve's error flag as read at a synchronising point, and clears it: resident launches end at once while
+// it is set, so a failure is reported by one call alone.
+gbfem_status report_solve_error(gbfem_handle h, int err)
+{
+	if (!err) return GBFEM_OK;
+	GB_CUDA(h, cudaMemsetAsync(h->d_pcgGlobal.p, 0, sizeof(PcgGlobal), h->stream));
+	return fail(h, GBFEM_CUDA_ERROR, err == 1 ? "persistent CG: grid barrier timed out"
+											  : "persistent CG: work share exceeded its shared-memory bound");
+}
+
 // Mixed-precision solve: one persistent launch, then its per-segment results are read back.
 gbfem_status run_mixed(gbfem_handle h, const double* b, double* x, int maxIter, bool timeSolve)
 {
@@ -1485,12 +1495,8 @@ gbfem_status run_mixed(gbfem_handle h, const double* b, double* x, int maxIter, 
 	GB_CUDA(h, cudaMemcpyAsync(h->h_seg, h->d_seg.p, sizeof(SegCtl) * nseg, cudaMemcpyDeviceToHost, st));
 	GB_CUDA(h, cudaMemcpyAsync(&g, h->d_pcgGlobal.p, sizeof(PcgGlobal), cudaMemcpyDeviceToHost, st));
 	GB_CUDA(h, cudaStreamSynchronize(st));
-	if (g.err)
-	{
-		GB_CUDA(h, cudaMemsetAsync(h->d_pcgGlobal.p, 0, sizeof(PcgGlobal), st));
-		return fail(h, GBFEM_CUDA_ERROR, g.err == 1 ? "persistent CG: grid barrier timed out"
-												  : "persistent CG: work share exceeded its shared-memory bound");
-	}
+	es = report_solve_error(h, g.err);
+	if (es != GBFEM_OK) return es;
 	if (timeSolve)
 	{
 		float ms = 0;
@@ -1506,10 +1512,7 @@ gbfem_status check_pcg_error(gbfem_handle h)
 {
 	PcgGlobal g;
 	GB_CUDA(h, cudaMemcpy(&g, h->d_pcgGlobal.p, sizeof(PcgGlobal), cudaMemcpyDeviceToHost));
-	if (g.err)
-		return fail(h, GBFEM_CUDA_ERROR, g.err == 1 ? "persistent CG: grid barrier timed out"
-												  : "persistent CG: work share exceeded its shared-memory bound");
-	return GBFEM_OK;
+	return report_solve_error(h, g.err);
 }
 
 // Hexahedra: the step's right-hand side from the stored K and block masses (x_t, v_t: the state the
@@ -1763,7 +1766,7 @@ gbfem_status step_graph(gbfem_handle h, double dt, int nsteps, uint32_t flags)
 	h->stats.steps += nsteps;
 	h->systemReady = true;
 	h->lastDt = dt;
-	if (acc[4 * (size_t)nseg + 1] != 0.0) return fail(h, GBFEM_CUDA_ERROR, "persistent CG: grid barrier timed out");
+	if (acc[4 * (size_t)nseg + 1] != 0.0) return report_solve_error(h, 1);
 	if (acc[4 * (size_t)nseg] != 0.0)
 	{
 		h->active = false;  // FemRepresentation.cpp:285-293
@@ -2888,7 +2891,7 @@ gbfem_status gbfem_rollout_forward(gbfem_handle h, double dt, int32_t nsteps, in
 	h->systemReady = true;
 	h->lastDt = dt;
 	const int nseg = (int)h->segNode.size() - 1;
-	if (acc[4 * (size_t)nseg + 1] != 0.0) return fail(h, GBFEM_CUDA_ERROR, "persistent CG: grid barrier timed out");
+	if (acc[4 * (size_t)nseg + 1] != 0.0) return report_solve_error(h, 1);
 	if (acc[4 * (size_t)nseg] != 0.0)
 	{
 		h->active = false;
@@ -3008,7 +3011,7 @@ gbfem_status gbfem_rollout_backward(gbfem_handle h, const double* lxT, const dou
 	h->stats.active = 1;
 	const int nseg = (int)h->segNode.size() - 1;
 	if (acc[4 * (size_t)nseg + 1] != 0.0 || adj[4 * (size_t)nseg + 1] != 0.0)
-		return fail(h, GBFEM_CUDA_ERROR, "persistent CG: grid barrier timed out");
+		return report_solve_error(h, 1);
 	if (acc[4 * (size_t)nseg] != 0.0) return fail(h, GBFEM_NONFINITE, "a re-run state is not finite");
 	if (h->stats.cg_max_iterations_hit > fwdHit || fwdHit > 0)
 		return fail(h, GBFEM_CG_MAXITER, "a solve of the reverse sweep did not converge");

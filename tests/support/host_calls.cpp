@@ -182,9 +182,12 @@ cudaError_t pcg_occupancy(int, int* n, size_t)
 	*n = 4;
 	return cudaSuccess;
 }
-cudaError_t pcg_launch(int form, const cudaLaunchConfig_t& cfg, const PcgArgs&)
+cudaError_t pcg_launch(int form, const cudaLaunchConfig_t& cfg, const PcgArgs& a)
 {
-	return (long long)cfg.dynamicSmemBytes > fake::limit(fake::pcg, form) ? cudaErrorInvalidValue : cudaSuccess;
+	if ((long long)cfg.dynamicSmemBytes > fake::limit(fake::pcg, form)) return cudaErrorInvalidValue;
+	for (int s = 0; s < a.nsegs && !fake::capturing; ++s) a.seg[s].converged = 1;
+	++fake::solves;
+	return cudaSuccess;
 }
 void launch_step_accumulate(const SegCtl*, int nseg, const int*, const int* err, double* acc, cudaStream_t)
 {
@@ -420,6 +423,45 @@ void failed_host_memory()
 	}
 }
 
+// A solve that gives up is reported by its own call; the next one starts with a clear flag (res_launch looks).
+void errors_reported_once()
+{
+	const Grid g(6, 6, 6);
+	const size_t n = g.X.size();
+	std::vector<double> b(3 * n, 1.0), x(3 * n), y(n), z(n), w(n);
+	gbfem_handle h = nullptr;
+	auto once = [&](auto f) {
+		fake::giveUp = true;
+		CHECK(f() == GBFEM_CUDA_ERROR);
+		fake::giveUp = false;
+		const int before = fake::solves;
+		CHECK(gbfem_step(h, 1e-3, 1, 0) == GBFEM_OK && fake::solves > before);
+		CHECK(f() == GBFEM_OK);
+	};
+	for (int precision : {GBFEM_PRECISION_FP64, GBFEM_PRECISION_MIXED})
+	{
+		const bool mixed = precision == GBFEM_PRECISION_MIXED;
+		gbfem_params p = params(precision, 0);
+		p.autotune = mixed;
+		CHECK(gbfem_create(&g.desc, &p, &h) == GBFEM_OK);
+		once([&] { return gbfem_step(h, 1e-3, 1, 0); });  // mixed: in the autotuner
+		if (mixed) CHECK(gbfem_set_tuning(h, 64, 4, 2, GBFEM_CG_ONE_PHASE) == GBFEM_OK);
+		once([&] { return gbfem_step(h, 1e-3, 1, 0); });
+		once([&] { return gbfem_apply_compliance(h, 3, b.data(), x.data(), 0, nullptr); });
+		once([&] {
+			return gbfem_adjoint_step(h, 1e-3, b.data(), b.data(), b.data(), b.data(), b.data(), y.data(), z.data(), w.data(),
+									  nullptr, 0);
+		});
+		if (mixed)
+		{
+			once([&] { return gbfem_step(h, 1e-3, 1, GBFEM_STEP_GRAPH); });
+			once([&] { return gbfem_rollout_forward(h, 1e-3, 4, 2, b.data(), b.data(), y.data(), z.data()); });
+			once([&] { return gbfem_rollout_backward(h, b.data(), b.data(), y.data(), z.data(), nullptr, nullptr); });
+		}
+		gbfem_destroy(h);
+	}
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -428,6 +470,7 @@ int main(int argc, char** argv)
 		{"two_devices", two_devices},
 		{"failed_allocations", failed_allocations},
 		{"failed_host_memory", failed_host_memory},
+		{"errors_reported_once", errors_reported_once},
 	};
 	const auto it = cases.find(argc > 1 ? argv[1] : "");
 	CHECK(it != cases.end());
