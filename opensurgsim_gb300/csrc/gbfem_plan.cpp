@@ -4,17 +4,23 @@
 
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <numeric>
 #include <utility>
 
 namespace gbfem {
 namespace {
 
-// Sorts indices by every third value from `coordinate`, then by index; the keys sit beside them for the sort.
+// Sorts indices by every third value from `coordinate`, then by index; the keys sit beside them for the sort. A node of no
+// element may lie anywhere, also at NaN, which has no place in an order: such nodes come last.
 void sort_along(const double* coordinate, int* first, int* last)
 {
 	std::vector<std::pair<double, int>> key(last - first);
-	for (int* i = first; i != last; ++i) key[i - first] = {coordinate[3 * (size_t)*i], *i};
+	for (int* i = first; i != last; ++i)
+	{
+		const double v = coordinate[3 * (size_t)*i];
+		key[i - first] = {std::isnan(v) ? std::numeric_limits<double>::infinity() : v, *i};
+	}
 	std::sort(key.begin(), key.end());
 	for (int* i = first; i != last; ++i) *i = key[i - first].second;
 }

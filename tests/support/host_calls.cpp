@@ -1,18 +1,22 @@
 // The host side of the C entry points (gbfem_host.cpp, gbfem_plan.cpp) on a stand-in for the CUDA runtime that
 // lives in host memory: two devices, allocations that can be made to fail, solves that can be made to report that
 // a wait ran out. Kernels do nothing. Runs the case named on the command line and prints "ok" or what went wrong.
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <limits>
 #include <map>
 #include <new>
+#include <random>
 #include <string>
 #include <vector>
 
 #include "../../include/gbfem.h"
 #include "gbfem_internal.h"
 #include "gbfem_pcg.h"
+#include "gbfem_plan.h"
 #include "gbfem_res.h"
 
 #define CHECK(x)                                              \
@@ -462,6 +466,41 @@ void errors_reported_once()
 	}
 }
 
+// Nodes of no element at NaN and at infinity: orders stay permutations that keep the others in theirs, and a body
+// with such nodes is created as before.
+void positions_without_an_order()
+{
+	const double nan = std::numeric_limits<double>::quiet_NaN(), inf = std::numeric_limits<double>::infinity();
+	std::mt19937 rng(1);
+	for (int trial = 0; trial < 60; ++trial)
+	{
+		const int n = 33 + (int)(rng() % 3000), every = 1 + trial % 7;
+		std::vector<double> X(3 * n);
+		for (double& v : X) v = rng() % every == 0 ? (rng() % 4 == 0 ? inf : nan) : rng() * 1e-9;
+		const std::vector<int> w(n, 5);
+		std::vector<int> seen(n, 0);
+		for (int i : gbfem::res_chunk_order(X, w)) ++seen.at(i);
+		for (const auto& part : gbfem::res_node_parts(X.data(), w, 1 + n / 200))
+			for (int i : part) ++seen.at(i);
+		for (int s : seen) CHECK(s == 2);
+		CHECK((int)gbfem::res_curve_keys(X.data(), n).size() == n);
+	}
+	for (int trial = 0; trial < 20; ++trial)
+	{
+		// Along a line, two parts: every number of the first lies before every one of the second.
+		const int n = 640;
+		std::vector<double> X(3 * n, 0.0);
+		for (int i = 0; i < n; ++i) X[3 * i] = rng() % 4 == 0 ? nan : rng() * 1e-9;
+		const auto parts = gbfem::res_node_parts(X.data(), std::vector<int>(n, 1), 2);
+		double last = -inf, first = inf;
+		for (int i : parts[0]) last = std::fmax(last, X[3 * i]);
+		for (int i : parts[1]) first = std::fmin(first, X[3 * i]);
+		CHECK(parts.size() == 2 && last <= first);
+	}
+	for (int precision : {GBFEM_PRECISION_FP64, GBFEM_PRECISION_MIXED})
+		for (double at : {nan, inf}) gbfem_destroy(create(Grid(9, 9, 9, 700, at), precision));
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -471,6 +510,7 @@ int main(int argc, char** argv)
 		{"failed_allocations", failed_allocations},
 		{"failed_host_memory", failed_host_memory},
 		{"errors_reported_once", errors_reported_once},
+		{"positions_without_an_order", positions_without_an_order},
 	};
 	const auto it = cases.find(argc > 1 ? argv[1] : "");
 	CHECK(it != cases.end());

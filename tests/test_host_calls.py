@@ -43,7 +43,8 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["two_devices", "failed_allocations", "failed_host_memory", "errors_reported_once"])
+@pytest.mark.parametrize("case", ["two_devices", "failed_allocations", "failed_host_memory", "errors_reported_once",
+                                  "positions_without_an_order"])
 def test_host_calls(program, case):
     out = subprocess.run([program, case], capture_output=True, text=True, env={**os.environ, "ASAN_OPTIONS": "detect_leaks=0"})
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout + out.stderr
