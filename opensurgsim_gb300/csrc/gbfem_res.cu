@@ -168,6 +168,7 @@ struct Shared
 	unsigned phases;
 	int task;
 	int mode;   // next phase: 0 CG step, 1 true residual, 2 rescale, 3 finished
+	int tiny;   // FP64: whether the solve runs on kUp times the right-hand side
 	float al, be, as, ratio;
 	double inv;   // 1 / s
 	double alpha, beta;
@@ -1307,6 +1308,9 @@ __device__ __forceinline__ void rows_mixed(const ResArgs& a, const ResPart p, un
 // Eigen's conjugate_gradient (Jacobi, zero start, |r|^2 < max(tol^2 |b|^2, DBL_MIN) before the iteration
 // is counted, iteration cap). p of the own and the halo rows is advanced in every CTA that uses it, from
 // the exchanged z; an iteration has two all-gathers (p.q, then |r|^2 and r.z).
+// 1 / r.z, formed while words travel, leaves FP64's range where r.z is below 1e-308 and |r|^2 not yet (right-hand
+// sides near 1e-150, a diagonal above one): such systems are solved for kUp times their right-hand side.
+constexpr double kUp = 0x1p400, kTinyNorm2 = 1e-150;
 template <int kForm, bool kCluster>
 __device__ __forceinline__ unsigned talk_f64(const ResArgs& a, const ResPart p, int rhs, unsigned base)
 {
@@ -1317,12 +1321,19 @@ __device__ __forceinline__ unsigned talk_f64(const ResArgs& a, const ResPart p, 
 	sums_wait();
 	total_f64<2>(a, T, ph, base + ph, v, [] {});
 	const double bb = v[0];
-	const double threshold = fmax(a.tol * a.tol * bb, DBL_MIN);
+	double threshold = fmax(a.tol * a.tol * bb, DBL_MIN);
 	double rz = v[1], rr = v[0];
 	int iter = 0, converged = 1;
 	int mode = (bb == 0.0 || bb < threshold || !isfinite(bb)) ? 3 : 0;
 	if (!isfinite(bb)) converged = 0;
 	if (given_up()) mode = 3;
+	const bool tiny = mode == 0 && bb < kTinyNorm2;
+	sh.tiny = tiny;
+	if (tiny)
+	{
+		threshold *= kUp * kUp;
+		rz *= kUp * kUp;
+	}
 	publish(mode);
 	while (mode != 3)
 	{
@@ -1370,6 +1381,7 @@ __device__ __forceinline__ unsigned talk_f64(const ResArgs& a, const ResPart p, 
 		if (lost) mode = 3;
 		publish(mode);
 	}
+	if (tiny) rr *= 1.0 / (kUp * kUp);
 	if (p.rank == 0 && (threadIdx.x & 31) == 0) write_result(a, p, rhs, bb, rr, iter, 0, converged, !isfinite(rr));
 	return ph;
 }
@@ -1421,6 +1433,15 @@ __device__ __forceinline__ void rows_f64(const ResArgs& a, const ResPart part_, 
 	sums_ready();
 	rows_sync();
 	scalars_wait();
+	if (sh.tiny)
+	{
+		for (int e = tid; e < nLoc; e += kRowThreads)
+		{
+			p[e] *= kUp;
+			if (e < nOwn) r[e] *= kUp;
+		}
+		rows_sync();
+	}
 #pragma unroll 1
 	while (sh.mode != 3)
 	{
@@ -1485,7 +1506,7 @@ __device__ __forceinline__ void rows_f64(const ResArgs& a, const ResPart part_, 
 	for (int e = tid; e < nOwn; e += kRowThreads)
 	{
 		const int I = a.perm[32 * S.c0 + e / bs];
-		if (I >= 0) xOut[(size_t)bs * I + e % bs] = x[e];
+		if (I >= 0) xOut[(size_t)bs * I + e % bs] = sh.tiny ? x[e] * (1.0 / kUp) : x[e];
 	}
 }
 
