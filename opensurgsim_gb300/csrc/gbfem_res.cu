@@ -105,6 +105,7 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e)
 }
 // Unevaluated pair h + l (~2^-46 relative). Sums and the CG scalars of the mixed form are held so: an
 // FP64 instruction takes 64 cycles of a scheduler here and an FP64 division 565 cycles.
+// The exponents are FP32's: talk_mixed scales what the matrix's units could put near its ends.
 struct Pair
 {
 	float h, l;
@@ -746,6 +747,7 @@ __device__ __forceinline__ unsigned talk_mixed(const ResArgs& a, const ResPart p
 	double bb[1], sD = 0.0, threshold, rrTrue;
 	Pair sP{}, alpha{1.f, 0.f}, rz{1.f, 0.f}, rzPend{}, ratioP{};
 	float rrLast = 0.f, thr32 = 0.f;
+	float unit = 1.f;  // what r.u and w.u are scaled by: 1 / r.u stays in FP32's range whatever the matrix's units
 	int iter = 0, updates = 0, converged = 0, nonfinite = 0, mode;
 	auto rescale = [&](double sNew) {  // r_true ~= s * r
 		sD = sNew;
@@ -808,6 +810,11 @@ __device__ __forceinline__ unsigned talk_mixed(const ResArgs& a, const ResPart p
 				rzInv = Pair{1.f, 0.f} / (mode == 2 ? rzPend * ratioP * ratioP : rz);
 				back = rzInv / alpha;
 			});
+			if (first && !(v[0].h > 0x1p-60f && v[0].h < 0x1p60f))
+				unit = __int_as_float(min(max(254 - ((__float_as_int(v[0].h) >> 23) & 255), 1), 253) << 23);
+			if (unit != 1.f)
+#pragma unroll
+				for (int k = 0; k < 2; ++k) v[k] = {unit * v[k].h, unit * v[k].l};
 			const Pair gN = pair(v[0].h, v[0].l), dN = pair(v[1].h, v[1].l);
 			const float rr = v[2].h + v[2].l;
 			if (mode == 0 && (rr < thr32 || rr < drop * rrLast || iter + 1 >= cap))

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import scipy.sparse as sp
 
-from opensurgsim_gb300 import _lib
+from opensurgsim_gb300 import _lib, mesh
 
 pytestmark = pytest.mark.gpu
 
@@ -27,3 +27,22 @@ def test_tiny_right_hand_sides(gpu_lib, scale, exponent):
     assert st == _lib.GBFEM_OK and 0 < it < 100
     r = np.linalg.norm(b - A @ (x * 10.0 ** -exponent))
     assert r <= max(1e-10 * np.linalg.norm(b), np.sqrt(2.3e-308) * 10.0 ** -exponent) + 1e-14 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("dims", [(3, 3, 4), (10, 10, 10), (11, 12, 30)])  # a cluster and more CTAs
+@pytest.mark.parametrize("exponent", [-90, -60, 60, 100, 110])
+def test_units_of_the_matrix(gpu_lib, dims, exponent):
+    """Density and Young's modulus times 2^k scale the mixed form's system by 2^k and leave its solution and
+    iterations. Both solves leave |b - S x| <= tol |b|, cond(S) below 5e3: 2 tol cond(S) of the velocities."""
+    from opensurgsim_gb300.body import Body
+
+    out = []
+    for k in (0, exponent):
+        s = mesh.scene_cube(*dims, seed=3, young=1e5 * 2.0 ** k, density=1000.0 * 2.0 ** k)
+        b = Body(s.mesh, gravity=(0, 0, -9.81), rayleigh_mass=0.01, rayleigh_stiffness=0.001, cg_tolerance=1e-10,
+                 precision=_lib.PRECISION_MIXED)
+        assert b.step(1e-3) == _lib.GBFEM_OK
+        out.append((b.stats()["cg_iterations"], b.state()[1]))
+        b.close()
+    assert out[0][0] == out[1][0]
+    assert np.linalg.norm(out[0][1] - out[1][1]) <= 2e-10 * 5e3 * np.linalg.norm(out[0][1])
