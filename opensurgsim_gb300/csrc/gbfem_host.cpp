@@ -1873,6 +1873,8 @@ void collect_segment_stats(gbfem_handle h)
 		ss[2] = std::min(ss[2], (double)c.converged);
 		ss[3] = std::max(ss[3], res);
 	}
+	// A single FP64 body reports a residual that is not a number as the launch-per-iteration CG does.
+	if (!h->persistent() && std::isnan(h->h_seg[0].rrTrue)) worst = h->h_seg[0].rrTrue;
 	h->stats.cg_relative_residual = worst;
 }
 
