@@ -2372,9 +2372,11 @@ gbfem_status compliance_resident(gbfem_handle h, ResDevice& d, int ncols, const 
 		}
 		for (int c = 0; c < k; ++c)
 		{
-			// The converging iteration counts here; a column below the threshold from the start has none.
+			// The last iteration counts here, whether it converged or broke down; a column below the threshold from the
+			// start or without a finite norm has none.
 			const double threshold = std::max(h->prm.cg_tolerance * h->prm.cg_tolerance * seg[c].bb, DBL_MIN);
-			*iterations += seg[c].iter + (seg[c].converged && seg[c].bb >= threshold ? 1 : 0);
+			const bool ended = seg[c].converged ? seg[c].bb >= threshold : (seg[c].nonfinite && std::isfinite(seg[c].bb));
+			*iterations += seg[c].iter + (ended ? 1 : 0);
 			*allConverged = *allConverged && seg[c].converged;
 		}
 	}

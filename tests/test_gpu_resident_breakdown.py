@@ -23,3 +23,20 @@ def test_residual_of_a_step_that_overflows(gpu_lib, flags):
     q = b.stats()
     b.close()
     assert np.isnan(q["cg_relative_residual"]) and q["cg_max_iterations_hit"] == 1 and q["refinement_sweeps"] == 0
+
+
+def test_iterations_of_columns_that_overflow(gpu_lib):
+    """r.z of the middle column is infinite: its first iteration gives NaN and is counted."""
+    b = _light(gravity=(0, 0, -9.81))
+    assert b.step(1e-3) == _lib.GBFEM_OK
+    B = np.random.default_rng(2).normal(size=(b.n, 3))
+    _, st, others = b.apply_compliance(B[:, ::2])
+    assert st == _lib.GBFEM_OK
+    B[:, 1] *= 1e151
+    X, st, it = b.apply_compliance(B)
+    assert st == _lib.GBFEM_CG_MAXITER and it == others + 1
+    assert np.isnan(X[:, 1]).any() and np.isfinite(X[:, ::2]).all()
+    B[:, 1] *= 1e10  # |b|^2 is infinite: no iteration
+    _, st, it = b.apply_compliance(B)
+    assert st == _lib.GBFEM_CG_MAXITER and it == others
+    b.close()
