@@ -838,7 +838,7 @@ __device__ __forceinline__ unsigned talk_mixed(const ResArgs& a, const ResPart p
 				sh.be = beta.h;
 				sh.as = (alpha * sP).h;
 				if (mode == 2) rrLast = rr;
-				if (!first) iter += 1;
+				if (!first && !nonfinite) iter += 1;  // one that cannot be taken is not counted
 				rz = gN;
 				mode = nonfinite ? 3 : 0;
 			}

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from opensurgsim_gb300 import _lib, mesh
+from opensurgsim_gb300.mesh import TetMesh
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +41,21 @@ def test_iterations_of_columns_that_overflow(gpu_lib):
     _, st, it = b.apply_compliance(B)
     assert st == _lib.GBFEM_CG_MAXITER and it == others
     b.close()
+
+
+def test_iterations_of_a_mixed_solve_that_breaks_down(gpu_lib):
+    """One free node whose 3x3 block is 2^40 times ones (the damping; the element's own part rounds away) and the
+    right-hand side 2^40 (1, 0, 0). In exact FP32: alpha = 1, r = (0, -1, -1), w.u = 4 = beta r.u / alpha, so the
+    second alpha is 2 / 0. The iteration that would have used it is not counted."""
+    from opensurgsim_gb300.body import Body
+
+    nodes = 0.01 * np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1.0]])
+    m = TetMesh(nodes, np.array([[0, 1, 2, 3]]), np.array([1e3]), np.array([0.4]), np.array([1000.0]),
+                np.arange(3, 12), (1, 1, 1), 0.01)
+    b = Body(m, gravity_enabled=False, cg_tolerance=1e-10, precision=_lib.PRECISION_MIXED)
+    b.set_tuning(64, 4, 2, _lib.CG_ONE_PHASE)
+    b.add_external_force(0, [1.0, 0, 0, 0], [2.0 ** 40, 0, 0], damping=2.0 ** 40 * np.ones((3, 3)))
+    b.step(1e-3)
+    q = b.stats()
+    b.close()
+    assert q["cg_max_iterations_hit"] == 1 and q["cg_iterations"] == 0
