@@ -14,7 +14,7 @@
 // 3.4 us for the grid). Every CTA of a system sums the same partials in the same order and takes
 // the same decisions; results do not depend on timing. A buffer written in phase k is written again in
 // phase k + 2, after its writer has every CTA's sums of phase k + 1, which each CTA sends after it
-// has used the words of phase k. Waits end after a wall-time limit (ResArgs::timeoutNs): the launch
+// has used the words of phase k. Waits end after a time limit (ResArgs::timeoutNs): the launch
 // then reports an error and returns.
 //
 // Systems of a batch are independent: each is solved by its own group of CTAs (as many as its matrix
@@ -71,25 +71,17 @@ __device__ __forceinline__ unsigned long long global_ns()
 	return t;
 }
 
-// Bound on one wait: after every 128 polls, whether another wait has given up or this one's wall time
-// has run out (then the launch's error flag is set). The time starts again while some system of the
-// launch still iterates (ResCtl::beat): a CTA may wait for another that is busy with an earlier system.
+// Bound on one wait: after every 128 polls, whether another wait has given up or this one's time has run out (then the
+// launch's error flag is set).
 struct Patience
 {
-	unsigned spins = 0, seen = 0;
-	unsigned long long t0 = 0;
+	unsigned spins = 0;
+	ResPatience time;
 	__device__ __forceinline__ bool lost(const ResArgs& a)
 	{
 		if ((++spins & 127u) != 0) return false;
-		const unsigned long long t = global_ns();
 		if (*(volatile int*)a.err) return true;
-		const unsigned beat = *(volatile unsigned*)&a.ctl->beat;
-		if (t0 == 0 || beat != seen)
-		{
-			t0 = t;
-			seen = beat;
-		}
-		if ((long long)(t - t0) <= a.timeoutNs) return false;
+		if (!time.over(global_ns(), *(volatile unsigned*)&a.ctl->beat, a.timeoutNs)) return false;
 		atomicExch(a.err, 1);
 		return true;
 	}

@@ -41,6 +41,28 @@ struct ResCtl
 	unsigned ticket;    // next entry of ResArgs::tasks
 };
 
+// How long a wait has polled. It begins again whenever some system of the launch has advanced (ResCtl::beat): a CTA may wait
+// for another that is busy with an earlier system. One poll counts for at most a sixteenth of the limit:
+// while the GPU runs another program the clock goes on and no CTA of this one does, and a wait that
+// is polled next after such a pause has not run out.
+struct ResPatience
+{
+	unsigned seen = 0;
+	bool begun = false;
+	unsigned long long last = 0;
+	long long waited = 0;
+	// At time t (ns): whether the limit is past.
+	__host__ __device__ bool over(unsigned long long t, unsigned beat, long long limit)
+	{
+		const long long step = (long long)(t - last), most = limit / 16;
+		waited = begun && beat == seen ? waited + (step < most ? step : most) : 0;
+		begun = true;
+		last = t;
+		seen = beat;
+		return waited >= limit;
+	}
+};
+
 struct ResArgs
 {
 	const ResPart* parts;

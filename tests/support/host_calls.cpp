@@ -501,6 +501,30 @@ void positions_without_an_order()
 		for (double at : {nan, inf}) gbfem_destroy(create(Grid(9, 9, 9, 700, at), precision));
 }
 
+// A wait's limit is polled time: one pause, however long, does not use it up; steady polling does, and progress
+// elsewhere begins it again.
+void patience()
+{
+	const long long limit = 1000000000, poll = 100000;
+	gbfem::ResPatience p;
+	unsigned long long t = 12345;
+	CHECK(!p.over(t, 7, limit));
+	CHECK(!p.over(t += 5 * limit, 7, limit));  // the GPU ran something else for five seconds
+	CHECK(!p.over(t += poll, 7, limit));
+	long long polls = 1;
+	while (!p.over(t += poll, 7, limit)) ++polls;
+	CHECK(polls * poll > limit / 2 && polls * poll < limit);
+	CHECK(!p.over(t += poll, 8, limit));  // some system advanced
+	for (int k = 1; k < limit / poll; ++k) CHECK(!p.over(t += poll, 8, limit));
+	CHECK(p.over(t += poll, 8, limit));
+	gbfem::ResPatience q;  // pauses alone end a wait all the same
+	int pauses = 0;
+	while (!q.over(t += 10 * limit, 0, limit)) ++pauses;
+	CHECK(pauses == 16);
+	gbfem::ResPatience r;  // a clock that begins at zero
+	CHECK(!r.over(0, 0, limit) && !r.over(limit, 0, limit));
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -511,6 +535,7 @@ int main(int argc, char** argv)
 		{"failed_host_memory", failed_host_memory},
 		{"errors_reported_once", errors_reported_once},
 		{"positions_without_an_order", positions_without_an_order},
+		{"patience", patience},
 	};
 	const auto it = cases.find(argc > 1 ? argv[1] : "");
 	CHECK(it != cases.end());

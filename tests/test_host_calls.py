@@ -44,7 +44,7 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("case", ["two_devices", "failed_allocations", "failed_host_memory", "errors_reported_once",
-                                  "positions_without_an_order"])
+                                  "positions_without_an_order", "patience"])
 def test_host_calls(program, case):
     out = subprocess.run([program, case], capture_output=True, text=True, env={**os.environ, "ASAN_OPTIONS": "detect_leaks=0"})
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout + out.stderr
