@@ -75,13 +75,13 @@ __device__ __forceinline__ unsigned long long global_ns()
 // launch's error flag is set).
 struct Patience
 {
-	unsigned spins = 0;
 	ResPatience time;
 	__device__ __forceinline__ bool lost(const ResArgs& a)
 	{
-		if ((++spins & 127u) != 0) return false;
+		if (!time.look()) return false;
+		const unsigned long long t = global_ns();
 		if (*(volatile int*)a.err) return true;
-		if (!time.over(global_ns(), *(volatile unsigned*)&a.ctl->beat, a.timeoutNs)) return false;
+		if (!time.over(t, *(volatile unsigned*)&a.ctl->beat, a.timeoutNs)) return false;
 		atomicExch(a.err, 1);
 		return true;
 	}

@@ -41,25 +41,27 @@ struct ResCtl
 	unsigned ticket;    // next entry of ResArgs::tasks
 };
 
-// How long a wait has polled. It begins again whenever some system of the launch has advanced (ResCtl::beat): a CTA may wait
-// for another that is busy with an earlier system. One poll counts for at most a sixteenth of the limit:
-// while the GPU runs another program the clock goes on and no CTA of this one does, and a wait that
-// is polled next after such a pause has not run out.
+// When a wait has run out: its limit is past on the clock and it has polled kResPolls times (1 ms and more), both since it
+// began or since some system of the launch last advanced (ResCtl::beat: a CTA may wait for another that is busy with an
+// earlier system). While the GPU runs another program the clock goes on and no CTA of this one does: a wait that
+// finds its limit past after such a pause is still polled.
+constexpr unsigned kResPolls = 2048;
 struct ResPatience
 {
-	unsigned seen = 0;
-	bool begun = false;
-	unsigned long long last = 0;
-	long long waited = 0;
-	// At time t (ns): whether the limit is past.
+	unsigned polls = 0, seen = 0;
+	unsigned long long t0 = 0;
+	// After a poll: whether to look at the time, after every 128.
+	__host__ __device__ bool look() { return (++polls & 127u) == 0; }
+	// At time t (ns): whether the wait has run out.
 	__host__ __device__ bool over(unsigned long long t, unsigned beat, long long limit)
 	{
-		const long long step = (long long)(t - last), most = limit / 16;
-		waited = begun && beat == seen ? waited + (step < most ? step : most) : 0;
-		begun = true;
-		last = t;
-		seen = beat;
-		return waited >= limit;
+		if (t0 == 0 || beat != seen)
+		{
+			t0 = t;
+			seen = beat;
+			polls = 0;
+		}
+		return polls >= kResPolls && (long long)(t - t0) > limit;
 	}
 };
 

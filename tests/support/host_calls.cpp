@@ -501,28 +501,31 @@ void positions_without_an_order()
 		for (double at : {nan, inf}) gbfem_destroy(create(Grid(9, 9, 9, 700, at), precision));
 }
 
-// A wait's limit is polled time: one pause, however long, does not use it up; steady polling does, and progress
-// elsewhere begins it again.
+// A wait runs out by the clock, but not at the end of a pause in which nothing ran; progress elsewhere begins it again.
 void patience()
 {
-	const long long limit = 1000000000, poll = 100000;
-	gbfem::ResPatience p;
+	const long long limit = 1000000000, poll = 1000;
 	unsigned long long t = 12345;
-	CHECK(!p.over(t, 7, limit));
-	CHECK(!p.over(t += 5 * limit, 7, limit));  // the GPU ran something else for five seconds
-	CHECK(!p.over(t += poll, 7, limit));
-	long long polls = 1;
-	while (!p.over(t += poll, 7, limit)) ++polls;
-	CHECK(polls * poll > limit / 2 && polls * poll < limit);
-	CHECK(!p.over(t += poll, 8, limit));  // some system advanced
-	for (int k = 1; k < limit / poll; ++k) CHECK(!p.over(t += poll, 8, limit));
-	CHECK(p.over(t += poll, 8, limit));
-	gbfem::ResPatience q;  // pauses alone end a wait all the same
-	int pauses = 0;
-	while (!q.over(t += 10 * limit, 0, limit)) ++pauses;
-	CHECK(pauses == 16);
-	gbfem::ResPatience r;  // a clock that begins at zero
-	CHECK(!r.over(0, 0, limit) && !r.over(limit, 0, limit));
+	auto polls = [&](gbfem::ResPatience& p, unsigned beat, long long most) {  // until it has run out, at most `most`
+		long long n = 0;
+		for (; n < most; ++n)
+		{
+			t += poll;
+			if (p.look() && p.over(t, beat, limit)) break;
+		}
+		return n;
+	};
+	gbfem::ResPatience p;
+	CHECK(polls(p, 7, 1000) == 1000);
+	t += 5 * limit;  // the GPU runs another program for five seconds
+	CHECK(polls(p, 7, 1000) == 1000);
+	CHECK(polls(p, 8, 1000) == 1000);  // some system advances
+	CHECK(polls(p, 8, limit / poll - 1000) == limit / poll - 1000);
+	const long long end = polls(p, 8, limit);
+	CHECK(end < 1300);  // the limit after the look that saw the advance
+	gbfem::ResPatience q;  // pauses alone
+	for (int k = 0; k < 2000; ++k, t += limit) CHECK(polls(q, 0, 1) == 1);
+	CHECK(polls(q, 0, limit) < 300);
 }
 
 }  // namespace
