@@ -334,6 +334,19 @@ GBFEM_API gbfem_status gbfem_last_error(gbfem_handle h, char* buf, size_t len);
 GBFEM_API gbfem_status gbfem_barrier_selftest(int32_t phases, int32_t stall, int64_t timeout_ns,
 											  int32_t* phases_passed, int64_t* max_wait_ns);
 
+/* Makes the waits of a handle's resident solves run out, to test their error path without a GPU fault: the solves
+ * of steps, adjoints and rollouts leave out the last share of a system, and every wait for it ends after wait_ns
+ * (in [1000, 1e9]) with GBFEM_CUDA_ERROR.
+ *   GBFEM_SOLVE_FAULT_NONE: solves as ever (wait_ns is not used);
+ *   GBFEM_SOLVE_FAULT_SHARE: the share never starts;
+ *   GBFEM_SOLVE_FAULT_ROWS: its first two sums are there, its rows are not (not inside a captured graph, and not
+ *     for a system whose shares form a cluster: there as GBFEM_SOLVE_FAULT_SHARE).
+ * GBFEM_INVALID_ARG where the handle's solves are not resident or the system that is drawn last has one share. */
+#define GBFEM_SOLVE_FAULT_NONE 0
+#define GBFEM_SOLVE_FAULT_SHARE 1
+#define GBFEM_SOLVE_FAULT_ROWS 2
+GBFEM_API gbfem_status gbfem_set_solve_fault(gbfem_handle h, int32_t fault, int64_t wait_ns);
+
 /* ---- LinearSparseSolveAndInverseCG on a caller matrix (LinearSparseSolveAndInverse.cpp:99-129).
  * Jacobi-preconditioned CG reading only the lower triangle (row >= col) of the CSC matrix, zero
  * initial guess, stop when |r|^2 < max(tol^2 |b|^2, DBL_MIN) or after max_iterations

@@ -38,6 +38,10 @@ COMPLIANCE_WARPING = 1
 CG_TWO_PHASE = 0
 CG_FP64 = 1
 CG_ONE_PHASE = 2
+# What gbfem_set_solve_fault leaves out of a handle's resident solves
+SOLVE_FAULT_NONE = 0
+SOLVE_FAULT_SHARE = 1
+SOLVE_FAULT_ROWS = 2
 
 # Every symbol the header declares; the CPU tests check the library exports all of them.
 EXPORTED = [
@@ -48,7 +52,7 @@ EXPORTED = [
     "gbfem_cg_destroy", "gbfem_cg_solve_noalloc", "gbfem_batch_create", "gbfem_batch_info",
     "gbfem_batch_segment_stats", "gbfem_set_materials_device", "gbfem_adjoint_step", "gbfem_get_tuning",
     "gbfem_set_tuning", "gbfem_apply_compliance", "gbfem_add_external_force", "gbfem_barrier_selftest",
-    "gbfem_set_solver_params", "gbfem_rollout_forward", "gbfem_rollout_backward",
+    "gbfem_set_solver_params", "gbfem_rollout_forward", "gbfem_rollout_backward", "gbfem_set_solve_fault",
 ]
 
 
@@ -161,6 +165,7 @@ def load():
         "gbfem_add_external_force": (S, [H, ctypes.c_int32, D, D, D, D]),
         "gbfem_barrier_selftest": (S, [ctypes.c_int32, ctypes.c_int32, ctypes.c_int64,
                                        ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int64)]),
+        "gbfem_set_solve_fault": (S, [H, ctypes.c_int32, ctypes.c_int64]),
         "gbfem_cg_solve_noalloc": (S, [ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                        ctypes.c_void_p, ctypes.c_void_p, ctypes.c_double, ctypes.c_int32,
                                        ctypes.c_void_p, ctypes.POINTER(ctypes.c_int32),

@@ -148,7 +148,8 @@ struct ResDevice
 	}
 	cudaError_t launch(const ResArgs& a, int ctas, cudaStream_t s) const
 	{
-		return res_launch(plan.form, std::min(ctas, a.nTasks), smem, a, s);
+		// A cluster has a CTA for every share, also for one that is left out (gbfem_set_solve_fault).
+		return res_launch(plan.form, cluster ? (int)plan.parts.size() : std::min(ctas, a.nTasks), smem, a, s);
 	}
 	void free()
 	{
@@ -340,6 +341,8 @@ struct gbfem_handle_s
 	ResExchange resLink;
 	int resBudget = 0;
 	float resNear = 1.f;  // ResArgs::nearFraction
+	int solveFault = GBFEM_SOLVE_FAULT_NONE;
+	long long solveWaitNs = kBarrierTimeoutNs;
 	int resForm() const { return res.ok ? res.form : (mixed() ? kResMixed : kResF64); }
 	DevBuf<float4> d_resOwn;  // kResMixedFar: p and x_delta of every row
 	// Compliance columns: plans by CTAs a column, their exchange, columns and results.
@@ -1362,6 +1365,27 @@ gbfem_status run_cg(gbfem_handle h, const double* b, double* x, int maxIter, boo
 // and the error against the FP64 path, and cut the step by 7%.
 constexpr double kRefreshDrop = 1e-5;
 
+// Leaves the share that is drawn last out of a launch (gbfem_set_solve_fault), and puts its sums of the first two
+// phases, zeros, into its system's mailboxes where that is asked for.
+gbfem_status leave_share_out(gbfem_handle h, ResArgs& a, bool capturing)
+{
+	a.nTasks -= 1;
+	if (h->solveFault != GBFEM_SOLVE_FAULT_ROWS || capturing || h->d_res.cluster) return GBFEM_OK;
+	const ResPart& p = h->res.parts[h->res.tasks[a.nTasks].x];
+	ResCtl ctl;
+	GB_CUDA(h, cudaMemcpyAsync(&ctl, a.ctl, sizeof(ResCtl), cudaMemcpyDeviceToHost, h->stream));
+	GB_CUDA(h, cudaStreamSynchronize(h->stream));
+	for (unsigned ph = 1; ph <= 2; ++ph)
+	{
+		const ResWord word{0u, 0u, 0u, ctl.epoch + ph}, words[2] = {word, word};
+		ResWord* box = a.mail + p.mail0 + (ph & 1u ? 2 * p.g * p.g : 0) + 2 * p.rank;
+		for (int consumer = 0; consumer < p.g; ++consumer)
+			GB_CUDA(h, cudaMemcpyAsync(box + 2 * (size_t)p.g * consumer, words, sizeof(words), cudaMemcpyHostToDevice, h->stream));
+	}
+	GB_CUDA(h, cudaStreamSynchronize(h->stream));
+	return GBFEM_OK;
+}
+
 // One resident solve of every system of the handle (gbfem_res.cu): one launch, no memory set before it.
 gbfem_status enqueue_resident(gbfem_handle h, const double* b, double* x, int maxIter, cudaEvent_t ev0, cudaEvent_t ev1,
 							  bool capturing)
@@ -1380,7 +1404,12 @@ gbfem_status enqueue_resident(gbfem_handle h, const double* b, double* x, int ma
 	a.tol = h->prm.cg_tolerance;
 	a.drop = kRefreshDrop;
 	a.nearFraction = h->resNear;
-	a.timeoutNs = kBarrierTimeoutNs;
+	a.timeoutNs = h->solveWaitNs;
+	if (h->solveFault != GBFEM_SOLVE_FAULT_NONE)
+	{
+		const gbfem_status fst = leave_share_out(h, a, capturing);
+		if (fst != GBFEM_OK) return fst;
+	}
 	a.seg = h->d_seg.p;
 	a.err = &h->d_pcgGlobal.p->err;
 	a.b = b;
@@ -2795,6 +2824,24 @@ void reset_call_stats(gbfem_handle h)
 }  // namespace
 
 extern "C" {
+
+gbfem_status gbfem_set_solve_fault(gbfem_handle h, int32_t fault, int64_t wait_ns)
+{
+	if (!h) return GBFEM_INVALID_ARG;
+	if (fault < GBFEM_SOLVE_FAULT_NONE || fault > GBFEM_SOLVE_FAULT_ROWS)
+		return fail(h, GBFEM_INVALID_ARG, "gbfem_set_solve_fault: unknown fault");
+	if (fault != GBFEM_SOLVE_FAULT_NONE)
+	{
+		if (wait_ns < 1000 || wait_ns > kBarrierTimeoutNs)
+			return fail(h, GBFEM_INVALID_ARG, "gbfem_set_solve_fault: wait_ns must be in [1000, 1e9]");
+		if (!h->resident() || h->res.parts[h->res.tasks.back().x].g == 1)
+			return fail(h, GBFEM_INVALID_ARG, "gbfem_set_solve_fault: no resident system of several shares");
+	}
+	h->solveFault = fault;
+	h->solveWaitNs = fault != GBFEM_SOLVE_FAULT_NONE ? wait_ns : kBarrierTimeoutNs;
+	h->tuneVersion++;  // captured graphs hold the launch's arguments
+	return GBFEM_OK;
+}
 
 gbfem_status gbfem_rollout_forward(gbfem_handle h, double dt, int32_t nsteps, int32_t checkpoint_every,
 								   const double* x0, const double* v0, double* xT, double* vT)

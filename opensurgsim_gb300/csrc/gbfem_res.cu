@@ -567,23 +567,27 @@ __device__ __forceinline__ bool receive_words(const ResArgs& a, const ResWord* b
 		if (16 * r < n) use(w[r]);
 	return true;
 }
+// Whether every CTA's 32 bytes of phase ph, the (ph - 1) / 2-th of its parity's barrier, are here.
+__device__ __forceinline__ bool arrived(unsigned ph)
+{
+	const unsigned bar = shared_address(&clusterBar[ph & 1]), parity = ((ph - 1) >> 1) & 1u;
+	unsigned done;
+	asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+				 : "=r"(done)
+				 : "r"(bar), "r"(parity)
+				 : "memory");
+	return done != 0u;
+}
 template <bool kCluster, typename F>
 __device__ __forceinline__ void receive(const ResArgs& a, const Talk<kCluster>& T, unsigned ph, unsigned tag, F use)
 {
 	const int lane = threadIdx.x & 31, j = lane & 15;
 	if constexpr (kCluster)
 	{
-		// Phase (ph - 1) / 2 of the parity's barrier: every CTA's 32 bytes are here.
-		const unsigned bar = shared_address(&clusterBar[ph & 1]), parity = ((ph - 1) >> 1) & 1u;
 		Patience wait;
 		for (;;)
 		{
-			unsigned done;
-			asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-						 : "=r"(done)
-						 : "r"(bar), "r"(parity)
-						 : "memory");
-			if (__all_sync(kFull, done)) break;
+			if (__all_sync(kFull, arrived(ph))) break;
 			if (__any_sync(kFull, wait.lost(a)))
 			{
 				sh.bad = 1;
@@ -611,6 +615,35 @@ __device__ __forceinline__ void receive(const ResArgs& a, const Talk<kCluster>& 
 		else
 			ok = receive_words<4>(a, from, n, tag, use);
 		if (!ok) return;
+	}
+}
+
+// After a solve whose waits gave up, the cluster's CTAs stand at different phases, at most one apart from the last that
+// all of them sent: words may still be on their way to a CTA that is done. The talking warp sends what its CTA has
+// not sent up to the last phase of any and waits until every word of the last phases has arrived. (A CTA sends in a
+// phase only when it has left the one before the last, so a barrier's phase is complete before its next arrival.)
+__device__ __noinline__ void settle_cluster()
+{
+	unsigned rank, g;
+	asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+	asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(g));
+	const unsigned sent = sh.phases;
+	unsigned most = 0;
+	for (unsigned j = 0; j < g; ++j)
+	{
+		unsigned theirs;
+		asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(theirs) : "r"(remote_address(shared_address(&sh.phases), (int)j)) : "memory");
+		most = max(most, theirs);
+	}
+	Talk<true> T{};
+	T.g = (int)g;
+	T.rank = (int)rank;
+	const unsigned long long t0 = global_ns();
+	for (unsigned ph = sent > 1u ? sent - 1u : 1u; ph <= most; ++ph)
+	{
+		if (ph > sent) send(T, ph, 0u, 0u, 0u, 0u);
+		while (!__all_sync(kFull, arrived(ph)))
+			if (__any_sync(kFull, global_ns() - t0 > 1000000000ull)) return;
 	}
 }
 
@@ -769,7 +802,7 @@ __device__ __forceinline__ unsigned talk_mixed(const ResArgs& a, const ResPart p
 		if (mode == 1)
 		{
 			double rr[1];
-			total_f64<1>(a, T, ph, base + ph, rr, [] {});
+			total_f64<1>(a, T, ph, base + ph, rr, [&] { lost = given_up(); });
 			rrTrue = rr[0];
 			updates += 1;
 			if (rrTrue < threshold)
@@ -1572,7 +1605,16 @@ __global__ void __launch_bounds__(kResThreads, 1) k_res(ResArgs a)
 		}
 	}
 	__syncthreads();
-	if (kCluster) cluster_sync();  // no CTA leaves while another may still write to it
+	if (kCluster)
+	{
+		cluster_sync();  // no CTA leaves while another may still write to it
+		if (*(volatile int*)a.err)  // the same answer in every CTA: whoever gave up did so before the barrier
+		{
+			if (threadIdx.x >= kRowThreads) settle_cluster();
+			__syncthreads();
+			cluster_sync();
+		}
+	}
 	// The last CTA to finish moves the tags past those of this launch.
 	if (threadIdx.x == 0)
 	{
