@@ -898,7 +898,12 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 		if (blocks * (h->mixed() ? 38 : 74) > 8LL * h->smCount * h->resBudget) resident = false;
 	}
 	gbfem_status ost = order_rows(h, X, !nodeOrder, resident, cost, so);
-	if (ost == GBFEM_OK && resident && !h->res.ok) ost = order_rows(h, X, false, false, cost, so);
+	if (resident && (ost != GBFEM_OK || !h->res.ok))
+	{
+		// No plan, or shares of mixed degrees padded the matrix past its indices: node order has the least padding.
+		h->err.clear();
+		ost = order_rows(h, X, false, false, cost, so);
+	}
 	if (ost != GBFEM_OK) return ost;
 	std::vector<int>&perm = so.perm, &segChunk = so.segChunk, &off = so.off, &scol = so.scol, &rcol = so.rcol,
 					&sellBase = so.sellBase;

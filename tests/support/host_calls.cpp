@@ -28,6 +28,8 @@
 		}                                                     \
 	while (0)
 
+long long fake_int32_max = 2147483647;  // INT32_MAX of the sources under test
+
 // ---- the stand-in -------------------------------------------------------------------------------------------------
 namespace fake {
 
@@ -528,6 +530,34 @@ void patience()
 	CHECK(polls(q, 0, limit) < 300);
 }
 
+// The order of the rows does not decide what is accepted: an FP64 batch, whose rows go into compact shares of about ten
+// chunks, needs no larger range of indices than a mixed one in node order.
+void index_range()
+{
+	std::vector<Grid> grids;
+	for (int k = 0; k < 70; ++k) grids.emplace_back(5, 6 + k % 3, 7);
+	std::vector<gbfem_mesh_desc> meshes;
+	for (const Grid& g : grids) meshes.push_back(g.desc);
+	auto accepted = [&](int precision) {
+		const gbfem_params p = params(precision, 0);
+		gbfem_handle h = nullptr;
+		const gbfem_status st = gbfem_batch_create((int)meshes.size(), meshes.data(), &p, &h);
+		if (h) gbfem_destroy(h);
+		return st == GBFEM_OK;
+	};
+	long long lo = 2000000, hi = 10000000;  // refused, accepted
+	while (hi - lo > 30000)
+	{
+		fake_int32_max = (lo + hi) / 2;
+		(accepted(GBFEM_PRECISION_MIXED) ? hi : lo) = fake_int32_max;
+	}
+	fake_int32_max = hi;
+	CHECK(lo > 2000000 && hi < 10000000);
+	CHECK(accepted(GBFEM_PRECISION_FP64));
+	fake_int32_max = lo;
+	CHECK(!accepted(GBFEM_PRECISION_FP64));
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -539,6 +569,7 @@ int main(int argc, char** argv)
 		{"errors_reported_once", errors_reported_once},
 		{"positions_without_an_order", positions_without_an_order},
 		{"patience", patience},
+		{"index_range", index_range},
 	};
 	const auto it = cases.find(argc > 1 ? argv[1] : "");
 	CHECK(it != cases.end());

@@ -25,7 +25,10 @@ def program(tmp_path_factory):
     sources = [os.path.join(CSRC, "gbfem_host.cpp"), os.path.join(CSRC, "gbfem_plan.cpp"),
                os.path.join(ROOT, "tests", "support", "host_calls.cpp")]
     objects = [os.path.join(out, os.path.basename(s) + ".o") for s in sources]
-    jobs = [subprocess.Popen(["g++", "-c", "-w", "-g", "-O0", "-std=c++17", "-fsanitize=address", "-I" + CSRC, "-I" + cuda, s,
+    limit = os.path.join(out, "limit.h")  # the range of 32-bit indices as a variable
+    with open(limit, "w") as f:
+        f.write("#include <cstdint>\n#undef INT32_MAX\nextern long long fake_int32_max;\n#define INT32_MAX fake_int32_max\n")
+    jobs = [subprocess.Popen(["g++", "-c", "-include", limit, "-w", "-g", "-O0", "-std=c++17", "-fsanitize=address", "-I" + CSRC, "-I" + cuda, s,
                               "-o", o]) for s, o in zip(sources, objects)]
     assert [j.wait() for j in jobs] == [0, 0, 0]
     symbols = {kind: set() for kind in "UT"}
@@ -44,7 +47,7 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("case", ["two_devices", "failed_allocations", "failed_host_memory", "errors_reported_once",
-                                  "positions_without_an_order", "patience"])
+                                  "positions_without_an_order", "patience", "index_range"])
 def test_host_calls(program, case):
     out = subprocess.run([program, case], capture_output=True, text=True, env={**os.environ, "ASAN_OPTIONS": "detect_leaks=0"})
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout + out.stderr
