@@ -224,13 +224,16 @@ def vector_passes(schedule):
     return 11 if schedule == 2 else 10
 
 
-def solve_roofline(schedule, traffic):
-    """Kernel, bound and DRAM traffic of the mixed solve. The one-phase schedule runs resident: its bytes are the
-    operands of its products, most of which shared memory and L2 serve, so their rate may pass HBM's."""
-    if schedule == 2:
+def solve_roofline(resident, traffic, achieved, peak):
+    """Kernel, bound, DRAM traffic and rate of the mixed solve. A resident solve's bytes are the operands of its products,
+    most of which shared memory and L2 serve: their rate is no fraction of HBM's. `traffic` was captured on the
+    persistent kernel."""
+    if resident:
         return {"kernel": "k_res (resident mixed solve, one launch per step)",
-                "bound": "on chip (operand bytes against the measured HBM rate)", "traffic": None}
-    return {"kernel": "k_pcg_persistent (persistent mixed solve, one launch per step)", "bound": "hbm", "traffic": traffic}
+                "bound": "on chip (operands from shared memory, L2 and HBM)", "traffic": None, "achieved": achieved,
+                "peak": peak, "unit": "GB/s", "frac": None}
+    return {"kernel": "k_pcg_persistent (persistent mixed solve, one launch per step)", "bound": "hbm", "traffic": traffic,
+            "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": (achieved / peak) if achieved else None}
 
 
 def bytes_per_iteration(nnz, N, s, vectors=10):
@@ -411,6 +414,7 @@ def run_batch(args, rank, world, local, dist):
     s = body.stats()
     launches = s["kernel_launches"]
     solve_ms = s["ms_spmv"]
+    resident = bool(s["resident"])
     ss = body.segment_stats()  # summed over the call's steps
     alg_bytes = float(np.dot(ss["iterations"], it_bytes) + np.dot(ss["refreshes"], rf_bytes)) + io_bytes * args.steps
     iters_total = int(ss["iterations"].max())
@@ -478,9 +482,8 @@ def run_batch(args, rank, world, local, dist):
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 2 * body.n * 8,
                 "d2h_bytes_per_step": 2 * body.n * 8},
         "roofline": {
-            **solve_roofline(tuning[3], load_traffic(f"pcg_persistent_batch{len(all_scenes)}") if world == 1 else None),
-            "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": (achieved / peak) if achieved else None,
+            **solve_roofline(resident, load_traffic(f"pcg_persistent_batch{len(all_scenes)}") if world == 1 else None,
+                             achieved, peak),
             "algorithmic_bytes_per_launch": per_launch, "avg_launch_ms": launch_ms,
             "peak_source": f"{peak_kind} (hbm_gbs)",
             "bytes_model": (f"per mesh: CG iterations x (nnz*4 + nnz/9*4 + 4(N+1) + {vpass}*4*3N) + refreshes x "
@@ -646,10 +649,13 @@ def run_single(args, rank, world, local, dist):
         vpass = vector_passes(body.tuning()[3])
         per_launch = (iters * bytes_per_iteration(body.nnz, body.num_nodes, 4, vpass)
                       + sweeps * bytes_per_refresh(body.nnz, body.num_nodes, 4) + 16 * body.n)
-        roof = solve_roofline(body.tuning()[3], load_traffic(f"pcg_persistent_{args.config}"))
         model = (f"CG iterations x (nnz*4 + nnz/9*4 + 4(N+1) + {vpass}*4*n) + refreshes x (nnz*4 + nnz/9*4 + 4(N+1) "
                  "+ 3*8*n) + 16n")
     achieved = per_launch / (launch_ms / 1e3) / 1e9 if launch_ms > 0 else None
+    if prec == _lib.PRECISION_FP64:
+        roof.update(achieved=achieved, peak=peak, unit="GB/s", frac=(achieved / peak) if achieved else None)
+    else:
+        roof = solve_roofline(bool(body.stats()["resident"]), load_traffic(f"pcg_persistent_{args.config}"), achieved, peak)
     line = {
         "metric": metric,
         "value": value,
@@ -677,8 +683,7 @@ def run_single(args, rank, world, local, dist):
         "clocks": clocks,
         "e2e": {"value": e2e_value, "unit": unit, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "roofline": {
-            **roof, "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": (achieved / peak) if achieved else None,
+            **roof,
             "algorithmic_bytes_per_launch": per_launch, "avg_launch_ms": launch_ms,
             "peak_source": f"{peak_kind} (hbm_gbs)", "bytes_model": model,
         },
@@ -794,6 +799,7 @@ def run_bar_full(args, rank, world, local, dist):
     peak, peak_kind = load_peak()
     am = agg["mixed"]
     solve_ms = am["ms_spmv"] / args.steps
+    resident = bool(bm.stats()["resident"])
     vpass = vector_passes(tuning[3])
     per_launch = (am["cg_iterations"] / args.steps * bytes_per_iteration(bm.nnz, bm.num_nodes, 4, vpass)
                   + am["refinement_sweeps"] / args.steps * bytes_per_refresh(bm.nnz, bm.num_nodes, 4) + 16 * bm.n)
@@ -827,10 +833,8 @@ def run_bar_full(args, rank, world, local, dist):
                 "d2h_bytes_per_step": 2 * bm.n * 8,
                 "how": f"{e2e_steps} hold steps after the timed run, host clock"},
         "roofline": {
-            **solve_roofline(tuning[3], load_traffic("pcg_persistent_bar")
-                             if abs(scene.mesh.h - BAR_H_WINDOW) < 1e-12 else None),
-            "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": (achieved / peak) if achieved else None,
+            **solve_roofline(resident, load_traffic("pcg_persistent_bar")
+                             if abs(scene.mesh.h - BAR_H_WINDOW) < 1e-12 else None, achieved, peak),
             "algorithmic_bytes_per_launch": per_launch, "avg_launch_ms": solve_ms,
             "peak_source": f"{peak_kind} (hbm_gbs)",
             "bytes_model": (f"CG iterations x (nnz*4 + nnz/9*4 + 4(N+1) + {vpass}*4*n) + refreshes x "

@@ -108,7 +108,7 @@ typedef struct gbfem_stats
 	int32_t active;
 	int32_t kernel_launches;        /* kernels this call launched */
 	int32_t spmv_timed;             /* CG matrix-vector launches timed (GBFEM_STEP_TIME_KERNELS) */
-	int32_t reserved0;
+	int32_t resident;               /* 1 where the handle's solves run resident (GBFEM_CG_ONE_PHASE below) */
 	double ms_spmv;                 /* summed device time of those launches (CUDA events) */
 	double reserved[2];
 } gbfem_stats;

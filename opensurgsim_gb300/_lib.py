@@ -105,7 +105,7 @@ class Stats(ctypes.Structure):
         ("active", ctypes.c_int32),
         ("kernel_launches", ctypes.c_int32),
         ("spmv_timed", ctypes.c_int32),
-        ("reserved0", ctypes.c_int32),
+        ("resident", ctypes.c_int32),
         ("ms_spmv", ctypes.c_double),
         ("reserved", ctypes.c_double * 2),
     ]

@@ -3194,6 +3194,7 @@ gbfem_status gbfem_get_stats(gbfem_handle h, gbfem_stats* out)
 {
 	if (!h || !out) return GBFEM_INVALID_ARG;
 	*out = h->stats;
+	out->resident = h->resident();
 	return GBFEM_OK;
 }
 

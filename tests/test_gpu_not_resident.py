@@ -144,3 +144,16 @@ def test_compliance_of_a_batch(gpu_lib, warping):
         assert st == _lib.GBFEM_OK
         assert np.linalg.norm(X[part] - x) <= 2e-8 * np.linalg.norm(X)
         one.close()
+
+
+def test_statistics_say_which_solve_runs(gpu_lib, hub):
+    cube = mesh.scene_cube(4, 4, 4).mesh
+    for m, precision, schedule, resident in ((hub, _lib.PRECISION_FP64, None, 0), (hub, _lib.PRECISION_MIXED, None, 0),
+                                             (cube, _lib.PRECISION_FP64, None, 1), (cube, _lib.PRECISION_MIXED, None, 1),
+                                             (cube, _lib.PRECISION_MIXED, _lib.CG_TWO_PHASE, 0),
+                                             ([hub, cube], _lib.PRECISION_FP64, None, 0), ([cube] * 3, _lib.PRECISION_FP64, None, 1)):
+        b, _ = _moving(m, precision)
+        if schedule is not None:
+            b.set_tuning(64, 4, 2, schedule)
+        assert b.step(1e-3) == _lib.GBFEM_OK and b.stats()["resident"] == resident
+        b.close()

@@ -51,3 +51,12 @@ def program(tmp_path_factory):
 def test_host_calls(program, case):
     out = subprocess.run([program, case], capture_output=True, text=True, env={**os.environ, "ASAN_OPTIONS": "detect_leaks=0"})
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout + out.stderr
+
+
+def test_the_benchmark_gives_no_hbm_fraction_of_a_resident_solve():
+    import bench
+
+    far = bench.solve_roofline(False, 123, 3000.0, 6000.0)
+    assert "k_pcg_persistent" in far["kernel"] and far["bound"] == "hbm" and far["frac"] == 0.5 and far["traffic"] == 123
+    near = bench.solve_roofline(True, 123, 9000.0, 6000.0)
+    assert "k_res" in near["kernel"] and near["frac"] is None and near["traffic"] is None and near["achieved"] == 9000.0
