@@ -1892,7 +1892,7 @@ gbfem_status apply_external(gbfem_handle h, double dt, const double* xt, cudaStr
 // Per-segment results of the last persistent solve (read back by run_mixed) into the statistics.
 void collect_segment_stats(gbfem_handle h)
 {
-	double worst = 0.0;
+	double worst = 0.0, last = 0.0;
 	for (int sg = 0; sg + 1 < (int)h->segNode.size(); ++sg)
 	{
 		const SegCtl& c = h->h_seg[sg];
@@ -1900,6 +1900,7 @@ void collect_segment_stats(gbfem_handle h)
 		h->stats.cg_iterations += c.iter;
 		h->stats.refinement_sweeps += c.updates;
 		worst = std::max(worst, res);
+		last = res;
 		if (!c.converged) h->stats.cg_max_iterations_hit++;
 		double* ss = &h->segStats[4 * (size_t)sg];
 		ss[0] += c.iter;
@@ -1907,9 +1908,9 @@ void collect_segment_stats(gbfem_handle h)
 		ss[2] = std::min(ss[2], (double)c.converged);
 		ss[3] = std::max(ss[3], res);
 	}
-	// A single FP64 body reports a residual that is not a number as the launch-per-iteration CG does.
-	if (!h->persistent() && std::isnan(h->h_seg[0].rrTrue)) worst = h->h_seg[0].rrTrue;
-	h->stats.cg_relative_residual = worst;
+	// A single FP64 body reports its residual as it is, also where it is not a number, as the launch-per-iteration CG does;
+	// the maximum over a batch's meshes leaves those out.
+	h->stats.cg_relative_residual = h->persistent() ? worst : last;
 }
 
 gbfem_status step_once(gbfem_handle h, double dt, uint32_t flags)

@@ -26,6 +26,20 @@ def test_residual_of_a_step_that_overflows(gpu_lib, flags):
     assert np.isnan(q["cg_relative_residual"]) and q["cg_max_iterations_hit"] == 1 and q["refinement_sweeps"] == 0
 
 
+@pytest.mark.parametrize("flags", [0, _lib.STEP_TIME_KERNELS])
+@pytest.mark.parametrize("value,residual", [(np.nan, 0.0), (np.inf, 0.0), (1e200, np.nan)])
+def test_residual_of_a_step_without_a_norm(gpu_lib, flags, value, residual):
+    """|b|^2 is not a number, where the residual is given as 0, or infinite, where it is infinity over infinity."""
+    b = _light()
+    v = np.zeros(b.n)
+    v[-1] = value
+    b.set_state(None, v)
+    b.step(1e-3, 1, flags)
+    q = b.stats()
+    b.close()
+    assert np.array_equal(q["cg_relative_residual"], residual, equal_nan=True) and q["cg_iterations"] == 0
+
+
 def test_iterations_of_columns_that_overflow(gpu_lib):
     """r.z of the middle column is infinite: its first iteration gives NaN and is counted."""
     b = _light(gravity=(0, 0, -9.81))
