@@ -890,8 +890,9 @@ gbfem_status build_body(gbfem_handle h, const gbfem_mesh_desc* m)
 	const bool nodeOrder = h->mixed() && chunks <= (nseg == 1 ? 1024 : 16384);
 	bool resident = !nodeOrder || chunks <= kOnePhaseChunksPerSlot * 4 * h->smCount;
 	// A system of eight times the chip's shared memory reads nearly all of its matrix from L2 and HBM in every
-	// product, which the other solves do with more loads in flight (63^3 hexahedra, mixed, 269 MB: 3.3 ms
-	// resident, 3.5 not).
+	// product, which the other solves do with more loads in flight. The sides do not meet at this line: resident is
+	// still the faster up to where the vectors stop fitting (steps of hexahedra, 63^3 mixed below it, 269 MB: solve 3.3 ms
+	// resident, 3.5 not; 65^3 above it: step 4.7 and 5.6 ms; 54^3 FP64: 5.6 and 11.8).
 	for (int sg = 0; sg < nseg; ++sg)
 	{
 		const int64_t blocks = h->adjPtr[h->segNode[sg + 1]] - h->adjPtr[h->segNode[sg]];
@@ -2282,7 +2283,8 @@ namespace {
 // Plan of ncols compliance columns as resident solves side by side, or null where none fits. A few CTAs
 // a column keep more columns going at once, many shorten each: an iteration takes about 6.5 us + 0.07 us a
 // weight of a share (FP64 sums at 64 cycles an instruction), and the columns go in waves. One plan per
-// number of CTAs, at most fifteen in a handle.
+// number of CTAs, at most fifteen in a handle, made by the first call that takes it (1,331 nodes, 1 to 160 columns: 0.2
+// to 0.4 ms on top of 0.5 to 5.9 ms).
 gbfem_status compliance_plan(gbfem_handle h, int ncols, ResDevice** out)
 {
 	*out = nullptr;

@@ -167,7 +167,9 @@ std::vector<int> res_widths(int form, double local, const std::vector<long long>
 	const int slot = res_layout(form, 1, 0).slotBytes;
 	const double room = smemBudget - (kResPieces * 32.0 * res_part_bytes(form) + 2048.0);
 	// Where CTAs are left over, shares shrink to this weight: below it an iteration is all exchange (mixed, 1,331
-	// nodes: 0.254 ms a solve at 40, 0.265 at 50, 0.279 at 80, 0.304 at 120; 216 nodes 0.230 at 40, 0.217 at 50;
+	// nodes: 0.254 ms a solve at 40, 0.265 at 50, 0.279 at 80, 0.304 at 120; whole steps in a graph at 40, 45, 50 and 60:
+	// 216 nodes 239, 239, 242, 242 us, 512 252, 252, 254, 273, 1,331 257, 263, 273, 273, 2,744 310, 298, 298, 298,
+	// 4,913 325, 328, 328, 335;
 	// FP64 1,331 nodes: 0.58 ms at 14, 0.65 at 20, 0.82 at 50; 17,280 scalar rows: 0.54 ms at 126, 0.50 at 250,
 	// 0.56 at 400). Past 128 CTAs the sums take a third poll (18,081 nodes: 0.415 ms on 128, 0.443 on 152; FP64
 	// 29,184 nodes 1.19 and 1.23).

@@ -1,5 +1,5 @@
 // Host check of the resident CG's plans (gbfem_plan.cpp) and of the slot and piece arithmetic the kernel does
-// with them (gbfem_res.cu, open_share / product / for_pieces), on random SELL matrices: every chunk in one
+// with them (gbfem_res.cu, open_share / open_mixed / product), on random SELL matrices: every chunk in one
 // share, local columns naming the right rows, shares within the shared memory, every slot multiplied once
 // (mixed: every chunk by one warp), cut chunks made of exactly their pieces, every share drawn once with its
 // system's others. Prints
